@@ -106,7 +106,9 @@ int lbm_get_stream(const lbm_sim* sim, void** cuda_stream);
  * (channel mode with f16 / bf16 storage; otherwise as 7).  Defaults: 3
  * for f32, 11 for f16 / bf16 (7 below 1024 columns), with rows_per_thread 8 for kernels 0 / 1 and a
  * band floor of 2 rows for the staged kernels; f64 storage always uses
- * kernel 0.  No counterpart in the reference, whose dispatch is fixed at
+ * kernel 0.  Until this is called, lbm_step takes three steps per launch
+ * where it can (channel mode below f64, 400,000 cells or more, no closure);
+ * the chosen kernel then takes every step by itself.  No counterpart in the reference, whose dispatch is fixed at
  * 256-wide 1-D workgroups (lbm.rs:102-106). */
 int lbm_set_tuning(lbm_sim* sim, int rows_per_thread, int kernel);
 
@@ -220,7 +222,7 @@ int lbm_step_rows(lbm_sim* sim, uint32_t y0, uint32_t y1, int flags);
 
 /* lbm_step replays CUDA graphs captured on first use: a call of 2 to 64
  * steps is captured whole and replayed by later calls of the same length;
- * longer calls replay runs of 16 steps (per buffer parity, recaptured when
+ * longer calls replay runs of 18 steps (per buffer parity, recaptured when
  * omega, the step kernel, the launch shape, the stream or the closure
  * change).  On by default; results are the same either way.  Not on the
  * legacy default stream, which cannot be captured, nor while the caller is

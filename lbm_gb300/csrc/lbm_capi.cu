@@ -12,6 +12,7 @@
 #include "../../include/lbm.h"
 #include "lbm_kernels.cuh"
 #include "lbm_stage.cuh"
+#include "lbm_multi.cuh"
 #include "lbm_closure.cuh"
 #include "lbm_closure_tc.cuh"
 #include "lbm_render.cuh"
@@ -50,6 +51,18 @@ int fail(int code, const char* fmt, ...) {
 constexpr int kBlockX = 128;
 constexpr int kReduceBlocks = 608;  // 4 x 152 SMs
 constexpr long long kPadCells = 4096;
+// Channel lattices of at least this many cells take three steps per launch
+// (k_step_multi).  Us per step against the one-step kernels, graph replays of
+// 64-step calls, f32 / f16: 512 x 256 5.4 against 4.0 / 4.7 against 4.1;
+// 768 x 384 5.3 against 5.5 / 4.75 against 4.9; 1024 x 512 5.9 against 8.0 /
+// 5.3 against 6.7; 2048 x 1024 15.5 against 26.7 / 12.1 against 14.4;
+// 4096 x 2048 47.3 against 94.0 / 37.4 against 51.9.  Below it a warp's row
+// latency (about 1 us, three dependent collisions) is not hidden.
+constexpr uint64_t kMultiCells = 400000;
+// With stochastic rounding a level costs a third more, and three lattices
+// stepping at once (each filling the other's gaps) were 4 % slower at
+// 1531 x 769 and 17 % faster at 2048 x 1024.
+constexpr uint64_t kMultiCellsSr = 1600000;
 
 size_t store_bytes(int storage) {
   switch (storage) {
@@ -66,7 +79,7 @@ namespace lbm_internal {
 void set_last_error(const char* msg) { g_err = msg; }
 }  // namespace lbm_internal
 
-constexpr int kStepGraph = 16;   // steps per captured graph (even)
+constexpr int kStepGraph = 18;   // steps per captured graph (even, whole three-step launches)
 constexpr int kRunGraphMax = 64; // longest call captured whole
 
 struct StepGraphKey {
@@ -77,13 +90,22 @@ struct StepGraphKey {
   cudaStream_t stream = nullptr;
   uint32_t sr_on = 0, sr_seed = 0;
   int sr_y0 = 0;
+  bool multi = false;  // three-step launches
   bool operator==(const StepGraphKey& o) const {
     return omega == o.omega && drift == o.drift && u_in == o.u_in && store_inlet == o.store_inlet &&
            kernel == o.kernel && rows == o.rows &&
            bands == o.bands &&
            staged_rows == o.staged_rows && closure == o.closure && stream == o.stream && sr_on == o.sr_on &&
-           sr_seed == o.sr_seed && sr_y0 == o.sr_y0;
+           sr_seed == o.sr_seed && sr_y0 == o.sr_y0 && multi == o.multi;
   }
+};
+
+// A captured run of steps.
+struct StepRun {
+  cudaGraphExec_t exec = nullptr;
+  StepGraphKey key;
+  uint32_t n = 0, launches = 0;  // steps; kernels per replay
+  bool flips = false;            // the two rest planes end up exchanged
 };
 
 struct lbm_sim {
@@ -109,6 +131,15 @@ struct lbm_sim {
   uint32_t* mask_d = nullptr;
   void* f_base[2] = {nullptr, nullptr};  // allocations
   void* rest_base = nullptr;
+  // the rest plane that a three-step launch writes (it then becomes `rest`),
+  // channel mode below f64 only
+  void* rest_out = nullptr;
+  void* rest_out_base = nullptr;
+  int rest_parity = 0;      // flips each time the two rest planes change places
+  bool inlet_same = true;   // both buffer sets hold the same words in column 0
+  bool tuned = false;       // lbm_set_tuning chose the step kernel
+  CUtensorMap planes[2] = {};  // the 8 planes of each buffer set, for its copies
+  int multi_occ = 0, multi_variant = -1;  // three-step kernel: CTAs per multiprocessor, for which variant
   void* mask_base = nullptr;
   void* mom = nullptr;  // rho, jx, jy planes
   int* flag_d = nullptr;
@@ -142,15 +173,12 @@ struct lbm_sim {
   float drift = 0.5f;
   bool closure_on = false;
   int closure_kernel = 0;  // 0: tensor cores (tcgen05), 1: CUDA cores
-  // captured runs of steps, one per buffer parity (lbm_step)
+  // captured runs of steps, one per buffer and rest-plane parity (lbm_step)
   bool use_graphs = true;
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};
-  StepGraphKey graph_key[2];
+  StepRun graph[4];
   // a whole call of n <= kRunGraphMax steps (the last one writing moments),
-  // per starting buffer parity: repeated calls of the same length replay it
-  cudaGraphExec_t run_graph[2] = {nullptr, nullptr};
-  StepGraphKey run_key[2];
-  uint32_t run_n[2] = {0, 0};
+  // per starting parity: repeated calls of the same length replay it
+  StepRun run_graph[4];
 };
 
 namespace {
@@ -314,6 +342,7 @@ int launch_init(lbm_sim* s, double rho, double ux, double uy, double amp, uint64
   s->cur = 0;
   s->materialised = true;
   s->moments_valid = false;
+  s->inlet_same = true;
   s->steps = 0;
   return reset_clock(s);
 }
@@ -343,15 +372,30 @@ int check_sim(const lbm_sim* s, bool pending_ok) {
 
 void release(lbm_sim* s) {
   for (auto& g : s->graph)
-    if (g) cudaGraphExecDestroy(g);
+    if (g.exec) cudaGraphExecDestroy(g.exec);
   for (auto& g : s->run_graph)
-    if (g) cudaGraphExecDestroy(g);
-  cudaFree(s->f_base[0]); cudaFree(s->f_base[1]); cudaFree(s->rest_base); cudaFree(s->mask_base); cudaFree(s->mom);
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+  cudaFree(s->f_base[0]); cudaFree(s->f_base[1]); cudaFree(s->rest_base); cudaFree(s->rest_out_base); cudaFree(s->mask_base); cudaFree(s->mom);
   cudaFree(s->flag_d); cudaFree(s->partial_d); cudaFree(s->staging_d); cudaFree(s->clock_d);
   cudaFree(s->closure_base); cudaFree(s->cnn_w); cudaFree(s->cnn_wpack); cudaFree(s->fallback_d);
   if (s->copied) cudaEventDestroy(s->copied);
   if (s->switched) cudaEventDestroy(s->switched);
   if (s->own_stream) cudaStreamDestroy(s->own_stream);
+}
+
+// Tensor maps of both buffer sets for the three-step kernel's copies.
+bool encode_maps(lbm_sim* s) {
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+      !fn)
+    return false;
+  for (int i = 0; i < 2; i++) {
+    const bool ok = s->es == 4 ? encode_planes<float>((EncodeTiledFn)fn, &s->planes[i], s->L, s->f[i])
+                               : encode_planes<__half>((EncodeTiledFn)fn, &s->planes[i], s->L, s->f[i]);
+    if (!ok) return false;
+  }
+  return true;
 }
 
 // Rows per band for `span` rows of W-column strips: as many bands as fit in
@@ -461,6 +505,84 @@ template <class St, int EDGE> int launch_staged_ns(lbm_sim* s, StepArgs<typename
   }
 }
 
+// Step arguments of a whole-lattice launch that reads buffer cur, writes
+// buffer `dst` and no moments.
+template <class S, class C> void fill_step_args(const lbm_sim* s, StepArgs<S, C>& a, int dst) {
+  a.L = s->L;
+  a.src = (const S*)s->f[s->cur];
+  a.dst = (S*)s->f[dst];
+  for (int p = 0; p < 8; p++) {
+    a.srcp[p] = a.src + (long long)p * s->L.ps;
+    a.dstp[p] = a.dst + (long long)p * s->L.ps;
+  }
+  a.rest = (S*)s->rest;
+  a.mask = s->mask_d;
+  a.omega = (C)s->omega;
+  a.materialised = s->materialised ? 1 : 0;
+  a.row0 = 0;
+  a.row_end = s->L.ny;
+  a.rho_out = a.jx_out = a.jy_out = nullptr;
+  a.flag = s->flag_d;
+  a.closure = s->closure_on ? s->closure_d : nullptr;
+  a.tau0 = 1.0f / s->omega;
+  a.drift = s->drift;
+  a.fallback = s->closure_on ? s->fallback_d : nullptr;
+  a.ref = store_ref(s);
+  a.sr.on = s->sr_on;
+  a.sr.seed = s->sr_seed;
+  a.sr.y0 = s->sr_y0;
+  a.sr.clock = s->sr_on ? s->clock_d : nullptr;
+  a.sr.t = s->clock_pending;
+}
+
+// Whether a call may take three steps in one launch: the lattice's default
+// kernel in channel mode, a state past its first step (a materialised one is
+// collided in place), uniform omega, and the same words in column 0 of both
+// buffer sets (the levels of a launch pull the inlet from one of them).
+bool multi_ok(const lbm_sim* s) {
+  return s->rest_out && !s->tuned && !s->materialised && !s->closure_on && s->inlet_same &&
+         (!s->sr_on || (uint64_t)s->L.nx * s->L.ny >= kMultiCellsSr);
+}
+
+int multi_key(const lbm_sim* s) { return s->sr_on ? 1 : 0; }
+
+// Three steps in one launch: reads buffer cur and `rest`, writes the other
+// buffer and `rest_out`; the caller updates the state.
+template <class St> int launch_multi(lbm_sim* s) {
+  using S = typename St::S;
+  using C = typename St::C;
+  using G = MultiGeom<S>;
+  MultiArgs<S, C> m;
+  fill_step_args(s, m.a, 1 - s->cur);
+  m.planes = s->planes[s->cur];
+  m.rest_out = (S*)s->rest_out;
+  m.one = 1.0f;
+  m.wcols = (s->L.nx + kMultiCols - 1) / kMultiCols;
+  auto kern = k_step_multi<St, false>;
+  if constexpr (St::kDev) {
+    if (s->sr_on) kern = k_step_multi<St, true>;
+  }
+  const size_t smem = (size_t)G::kStages * G::kBytes;
+  const int variant = multi_key(s);
+  if (s->multi_variant != variant) {
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int occ = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32, smem));
+    if (occ < 1) return fail(LBM_ERR_CUDA, "three-step kernel does not fit on a multiprocessor");
+    s->multi_occ = occ;
+    s->multi_variant = variant;
+  }
+  // one wave of bands where that leaves 8 to 24 rows each: shorter bands
+  // repeat too many halo rows (2048 x 1024, f32: 16 rows 47 us a launch, 4 rows
+  // 58), taller ones wait for their last warp (4096 x 2048: 24 rows in 2.4
+  // waves 143, 59 rows in one wave 153)
+  const int bands = std::max(1, s->multi_occ * s->sms / m.wcols);
+  m.a.rows = std::min(std::max((s->L.ny + bands - 1) / bands, 8), 24);
+  kern<<<m.wcols * ((s->L.ny + m.a.rows - 1) / m.a.rows), 32, smem, s->stream>>>(m);
+  CK_LAUNCH();
+  return LBM_OK;
+}
+
 int compute_moments(lbm_sim* s) {
   dim3 grid((s->L.nx + kBlockX - 1) / kBlockX, s->L.ny);
   auto launch = [&](auto tag) -> int {
@@ -541,6 +663,14 @@ int lbm_create(uint32_t nx, uint32_t ny, float omega, int edge_mode, int storage
   if ((rc = alloc_padded(&s->rest_base, &s->rest, (size_t)s->L.ps, s->es))) return rc;
   if ((rc = alloc_padded(&s->mask_base, (void**)&s->mask_d, (size_t)s->L.mw * ny, 4))) return rc;
   (void)plane;
+  if (edge_mode == EDGE_CHANNEL && storage != STORE_F64 && (uint64_t)nx * ny >= kMultiCells) {
+    if ((rc = alloc_padded(&s->rest_out_base, &s->rest_out, (size_t)s->L.ps, s->es))) return rc;
+    if (!encode_maps(s)) {
+      release(s);
+      delete s;
+      return fail(LBM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    }
+  }
   if ((rc = alloc(&s->mom, 3 * (size_t)s->L.ps * s->cs))) return rc;
   if ((rc = alloc((void**)&s->flag_d, 4))) return rc;
   if ((rc = alloc((void**)&s->partial_d, (size_t)kReduceBlocks * 3 * 8))) return rc;
@@ -622,6 +752,7 @@ int lbm_set_tuning(lbm_sim* s, int rows_per_thread, int kernel) {
   if (kernel < 0 || kernel > 13) return fail(LBM_ERR_ARG, "kernel %d", kernel);
   s->rows = rows_per_thread;
   s->kernel = kernel;
+  s->tuned = true;
   s->staged_variant = -1;  // recompute the staged launch shape
   return LBM_OK;
 }
@@ -722,7 +853,10 @@ int lbm_set_inlet_velocity(lbm_sim* s, float ux, int reset_field) {
     return LBM_OK;
   };
   rc = dispatch_storage(s->storage, launch);
-  if (!rc) s->launches++;
+  if (!rc) {
+    s->launches++;
+    s->inlet_same = true;
+  }
   return rc;
 }
 
@@ -831,40 +965,18 @@ static int launch_rows(lbm_sim* s, bool last, int row0, int row_end, int dst) {
   // would spill its doubled register footprint.
   const int variant = s->storage == STORE_F64 ? 0 : s->kernel;
   dim3 grid((s->L.nx + kBlockX - 1) / kBlockX, (row_end - row0 + rows - 1) / rows);
-  const int src = s->cur;
   auto launch = [&](auto tag) -> int {
     using St = decltype(tag);
     using S = typename St::S;
     using C = typename St::C;
     StepArgs<S, C> a;
-    a.L = s->L;
-    a.src = (const S*)s->f[src];
-    a.dst = (S*)s->f[dst];
-    for (int p = 0; p < 8; p++) {
-      a.srcp[p] = a.src + (long long)p * s->L.ps;
-      a.dstp[p] = a.dst + (long long)p * s->L.ps;
-    }
-    a.rest = (S*)s->rest;
-    a.mask = s->mask_d;
-    a.omega = (C)s->omega;
-    a.materialised = s->materialised ? 1 : 0;
+    fill_step_args(s, a, dst);
     a.rows = rows;
     a.row0 = row0;
     a.row_end = row_end;
     a.rho_out = last ? (C*)mom_plane(s, 0) : nullptr;
     a.jx_out = last ? (C*)mom_plane(s, 1) : nullptr;
     a.jy_out = last ? (C*)mom_plane(s, 2) : nullptr;
-    a.flag = s->flag_d;
-    a.closure = s->closure_on ? s->closure_d : nullptr;
-    a.tau0 = 1.0f / s->omega;
-    a.drift = s->drift;
-    a.fallback = s->closure_on ? s->fallback_d : nullptr;
-    a.ref = store_ref(s);
-    a.sr.on = s->sr_on;
-    a.sr.seed = s->sr_seed;
-    a.sr.y0 = s->sr_y0;
-    a.sr.clock = s->sr_on ? s->clock_d : nullptr;
-    a.sr.t = s->clock_pending;
     if (variant >= 2) {
       return s->edge == EDGE_REF ? launch_staged_ns<St, EDGE_REF>(s, a) : launch_staged_ns<St, EDGE_CHANNEL>(s, a);
     } else if (variant == 1) {
@@ -895,6 +1007,40 @@ static int launch_step(lbm_sim* s, bool last) {
   return LBM_OK;
 }
 
+static void swap_rest(lbm_sim* s) {
+  std::swap(s->rest, s->rest_out);
+  s->rest_parity ^= 1;
+}
+
+// Three steps in one launch, without moments.
+static int launch_steps3(lbm_sim* s) {
+  auto launch = [&](auto tag) -> int {
+    using St = decltype(tag);
+    if constexpr (sizeof(typename St::S) <= 4) return launch_multi<St>(s);
+    else return fail(LBM_ERR_ARG, "bad storage %d", s->storage);
+  };
+  int rc = dispatch_storage(s->storage, launch);
+  if (rc) return rc;
+  s->launches++;
+  s->cur = 1 - s->cur;
+  swap_rest(s);
+  s->steps += kMultiSteps;
+  if (s->sr_on) s->clock_pending += kMultiSteps;
+  return LBM_OK;
+}
+
+// The next launch of a call with `left` steps to go: three steps where that
+// is possible and a single step is left to end the call (it writes the
+// moments, and the other buffer then holds the step before it as ever).
+static int launch_some(lbm_sim* s, uint32_t left, bool moments, uint32_t* taken) {
+  if (left > (uint32_t)kMultiSteps - (moments ? 0u : 1u) && multi_ok(s)) {
+    *taken = kMultiSteps;
+    return launch_steps3(s);
+  }
+  *taken = 1;
+  return launch_step(s, moments && left == 1);
+}
+
 // Everything a captured run of steps depends on besides the buffers.
 static StepGraphKey graph_key(const lbm_sim* s) {
   StepGraphKey k;
@@ -911,6 +1057,7 @@ static StepGraphKey graph_key(const lbm_sim* s) {
   k.sr_on = s->sr_on;
   k.sr_seed = s->sr_seed;
   k.sr_y0 = s->sr_y0;
+  k.multi = multi_ok(s);
   return k;
 }
 
@@ -926,39 +1073,61 @@ static int advance_clock(lbm_sim* s) {
 
 static void drop_step_graphs(lbm_sim* s) {
   for (auto* gs : {s->graph, s->run_graph})
-    for (int i = 0; i < 2; i++)
-      if (gs[i]) {
-        cudaGraphExecDestroy(gs[i]);
-        gs[i] = nullptr;
+    for (int i = 0; i < 4; i++)
+      if (gs[i].exec) {
+        cudaGraphExecDestroy(gs[i].exec);
+        gs[i].exec = nullptr;
       }
 }
 
-// Capture n steps from the current buffer parity into `out`; with
-// `moments` the last one writes the moments.
-static int capture_steps(lbm_sim* s, cudaGraphExec_t& out, uint32_t n, bool moments) {
-  if (out) {
-    cudaGraphExecDestroy(out);
-    out = nullptr;
+// Capture n steps from the current parity into `run`; with `moments` the
+// last one writes the moments.
+static int capture_steps(lbm_sim* s, StepRun& run, uint32_t n, bool moments) {
+  if (run.exec) {
+    cudaGraphExecDestroy(run.exec);
+    run.exec = nullptr;
   }
-  const int cur0 = s->cur;
-  const uint64_t steps0 = s->steps, launches0 = s->launches;
+  const int cur0 = s->cur, rest0 = s->rest_parity;
   int rc = advance_clock(s);  // the run's launches count from the clock as it stands
   if (rc) return rc;
+  const uint64_t steps0 = s->steps, launches0 = s->launches;
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-  for (uint32_t k = 0; k < n && !rc; k++) rc = launch_step(s, moments && k + 1 == n);
+  for (uint32_t k = 0, took = 0; k < n && !rc; k += took) rc = launch_some(s, n - k, moments, &took);
   if (!rc) rc = advance_clock(s);  // recorded: every replay advances the clock by n
   s->clock_pending = 0;
   const cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+  run.launches = (uint32_t)(s->launches - launches0);
+  run.flips = s->rest_parity != rest0;
+  run.n = n;
+  run.key = graph_key(s);
   s->cur = cur0;  // the capture recorded the launches without running them
+  if (run.flips) swap_rest(s);
   s->steps = steps0;
   s->launches = launches0;
   s->materialised = false;
   if (rc) return rc;
   if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "stream capture: %s", cudaGetErrorString(e));
-  const cudaError_t ei = cudaGraphInstantiate(&out, g, 0);
+  const cudaError_t ei = cudaGraphInstantiate(&run.exec, g, 0);
   cudaGraphDestroy(g);
   if (ei != cudaSuccess) return fail(LBM_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ei));
+  return LBM_OK;
+}
+
+// Replay n steps from the current parity, captured first where `runs` holds
+// no such run.
+static int replay_steps(lbm_sim* s, StepRun* runs, uint32_t n, bool moments) {
+  StepRun& run = runs[s->cur + 2 * s->rest_parity];
+  int rc;
+  if (!run.exec || run.n != n || !(run.key == graph_key(s))) {
+    if ((rc = capture_steps(s, run, n, moments))) return rc;
+  }
+  if ((rc = advance_clock(s))) return rc;
+  CK(cudaGraphLaunch(run.exec, s->stream));
+  s->steps += n;
+  s->launches += run.launches;
+  s->cur ^= (int)(n & 1u);
+  if (run.flips) swap_rest(s);
   return LBM_OK;
 }
 
@@ -966,7 +1135,7 @@ int lbm_step(lbm_sim* s, uint32_t n) {
   CHECK_SIM(s);
   if (n == 0) return LBM_OK;
   // Launch overhead dominates small grids, so steps replay captured graphs
-  // once the launch shape is known (the legacy default stream cannot be
+  // once the launch shapes are known (the legacy default stream cannot be
   // captured): a short call repeated with the same length replays one graph
   // of the whole call; longer calls replay runs of kStepGraph steps.
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;  // a caller's own capture: plain launches
@@ -974,44 +1143,23 @@ int lbm_step(lbm_sim* s, uint32_t n) {
   auto steady = [&]() {
     return s->use_graphs && s->stream != nullptr && capturing == cudaStreamCaptureStatusNone && !s->materialised &&
            (s->storage == STORE_F64 || s->kernel < 2 ||
-            s->staged_variant == staged_key(s->kernel, s->closure_on, s->sr_on != 0u));
+            s->staged_variant == staged_key(s->kernel, s->closure_on, s->sr_on != 0u)) &&
+           (n <= (uint32_t)kMultiSteps || !multi_ok(s) || s->multi_variant == multi_key(s));
   };
   if (n >= 2 && n <= (uint32_t)kRunGraphMax && steady()) {
-    const int c = s->cur;
-    if (!s->run_graph[c] || s->run_n[c] != n || !(s->run_key[c] == graph_key(s))) {
-      int rc = capture_steps(s, s->run_graph[c], n, true);
-      if (rc) return rc;
-      s->run_key[c] = graph_key(s);
-      s->run_n[c] = n;
-    }
-    int rc = advance_clock(s);
-    if (rc) return rc;
-    CK(cudaGraphLaunch(s->run_graph[c], s->stream));
-    s->steps += n;
-    s->launches += n + (s->sr_on ? 1 : 0);
-    s->cur = c ^ (int)(n & 1u);
-    s->moments_valid = true;
-    return LBM_OK;
+    int rc = replay_steps(s, s->run_graph, n, true);
+    if (!rc) s->moments_valid = true;
+    return rc;
   }
-  for (uint32_t k = 0; k < n;) {
-    const uint32_t left = n - k;
-    if (left > (uint32_t)kStepGraph && steady()) {
-      if (!s->graph[s->cur] || !(s->graph_key[s->cur] == graph_key(s))) {
-        int rc = capture_steps(s, s->graph[s->cur], kStepGraph, false);
-        if (rc) return rc;
-        s->graph_key[s->cur] = graph_key(s);
-      }
-      int rc = advance_clock(s);
-      if (rc) return rc;
-      CK(cudaGraphLaunch(s->graph[s->cur], s->stream));
-      s->steps += kStepGraph;  // even: the buffer parity is unchanged
-      s->launches += kStepGraph + (s->sr_on ? 1 : 0);
-      k += kStepGraph;
-      continue;
+  for (uint32_t k = 0, took = 0; k < n; k += took) {
+    int rc;
+    if (n - k > (uint32_t)kStepGraph && steady()) {
+      rc = replay_steps(s, s->graph, kStepGraph, false);
+      took = kStepGraph;
+    } else {
+      rc = launch_some(s, n - k, true, &took);
     }
-    int rc = launch_step(s, k + 1 == n);
     if (rc) return rc;
-    k++;
   }
   int rc = advance_clock(s);
   if (rc) return rc;
@@ -1177,6 +1325,7 @@ static int write_pops(lbm_sim* s, const void* in, bool f64) {
   s->cur = 0;
   s->materialised = true;
   s->moments_valid = false;
+  s->inlet_same = true;
   s->steps = 0;
   return reset_clock(s);
 }
@@ -1661,6 +1810,9 @@ int lbm_checkpoint_load(lbm_sim* s, const void* buf, size_t len) {
   s->cur = (int)h.cur;
   s->materialised = h.materialised != 0;
   s->moments_valid = false;
+  s->inlet_same = true;  // column 0 of the two buffer sets
+  for (size_t row = 0; row < 8 * (size_t)s->L.ny && s->inlet_same; row++)
+    s->inlet_same = std::memcmp(q + row * s->L.nx * e, q + (8 * cells + row * s->L.nx) * e, e) == 0;
   return reset_clock(s);
 }
 
@@ -1707,6 +1859,7 @@ static int rows_io(lbm_sim* s, uint32_t y, uint32_t nrows, uint32_t slot_mask, v
   const cudaMemcpyKind kind = read ? (on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost)
                                    : (on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
   char* buf = (char*)host;
+  if (!read) s->inlet_same = false;  // column 0 of one buffer set only
   for (int slot = 0; slot < 8; slot++) {
     if (!((slot_mask >> slot) & 1u)) continue;
     // while a step taken in row ranges is incomplete: the buffer it writes
