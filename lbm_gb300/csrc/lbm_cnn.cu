@@ -38,191 +38,457 @@ int cfail(int code, const char* fmt, ...) {
   } while (0)
 
 constexpr int kRow = 128;          // pixels per block in the per-pixel kernels
-constexpr int kWTile = 64;         // pixels per tile in the weight-gradient kernel
-constexpr int kWBlocks = 304;      // weight-gradient blocks (2 per SM)
+constexpr int kTile = 64;          // pixels of a row in a convolution tile
+constexpr int kTileS = 72;         // a staged row: columns x0 - 4 .. x0 + 67 of the tile at x0, whole 16-byte words
+constexpr int kTile0 = 4;          // index of column x0 in it
+constexpr int kChunk = 8;          // input channels staged at a time
+constexpr int kWBlocks = 304;      // partial sums the weight gradient's scratch holds
 constexpr int kMaxC = 32;          // channels handled by the templates
 constexpr int kLossBlocks = 608;   // loss partial sums (4 per SM)
 
 inline cudaStream_t as_stream(void* s) { return (cudaStream_t)s; }
 
-// ---- forward: one thread per output pixel, all COUT channels --------------------
-template <int COUT>
-__global__ void __launch_bounds__(kRow) k_conv_fwd(const float* __restrict__ x, int CIN, int H, int W,
-                                                   const float* __restrict__ w, const float* __restrict__ b, int relu,
-                                                   float* __restrict__ y) {
-  extern __shared__ float4 sw4[];
-  float* sw = (float*)sw4;  // [CIN * 9][COUT]
-  for (int i = threadIdx.x; i < CIN * 9 * COUT; i += blockDim.x) {
-    const int co = i % COUT, r = i / COUT;
-    sw[i] = w[co * CIN * 9 + r];
+__device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
+
+// Asynchronous 4-byte copy to shared memory, zero where `in` is false (the
+// address is then not read).
+__device__ __forceinline__ void copy4(float* dst, const float* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 4 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 16 : 0)
+               : "memory");
+}
+// One staged row by one warp: columns x0 - 1 .. x0 + 64 of the image row at
+// `src` (zero where row_in is false or outside [0, W)).  `wide` (W a multiple of
+// four, 16-byte aligned rows): 18 copies of four columns, each wholly inside or outside.
+__device__ __forceinline__ void stage_row(float* dst, const float* src, bool row_in, int x0, int W, bool wide) {
+  const int lane = threadIdx.x & 31;
+  if (wide) {
+    const int xx = x0 - kTile0 + 4 * lane;
+    const bool in = row_in && xx >= 0 && xx < W;
+    if (lane < kTileS / 4) copy16(dst + 4 * lane, src + (in ? xx : 0), in);
+    return;
   }
-  __syncthreads();
-  const int px = blockIdx.x * kRow + threadIdx.x;
-  const int n = blockIdx.y / H, py = blockIdx.y % H;
-  if (px >= W) return;
-  const size_t plane = (size_t)H * W;
-  float acc[COUT];
 #pragma unroll
-  for (int co = 0; co < COUT; co++) acc[co] = b[co];
-  const float* xn = x + (size_t)n * CIN * plane;
-  for (int ci = 0; ci < CIN; ci++) {
-    const float* xc = xn + ci * plane;
+  for (int k = 0; k < 3; k++) {
+    const int j = lane + 32 * k, xx = x0 - 1 + j;
+    const bool in = row_in && xx >= 0 && xx < W;
+    if (j < kTile + 2) copy4(dst + kTile0 - 1 + j, src + (in ? xx : 0), in);
+  }
+}
+__host__ __device__ __forceinline__ bool wide_rows(const float* p, const float* q, int W) {
+  return W % 4 == 0 && (((uintptr_t)p | (uintptr_t)q) & 15u) == 0;
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Starts the copies of rows y0 - 1 .. y0 + rows of channels c0 .. c0 + nc - 1
+// of image n into `sx` [nc][rows + 2][kTileS].  mask_staged visits the same
+// elements by the same threads, so a thread may use what it copied itself
+// without a barrier.
+__device__ __forceinline__ void stage_rows(const float* __restrict__ x, int n, int C, int c0, int nc, int H, int W,
+                                           int x0, int y0, int rows, bool wide, float* sx) {
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  for (int r = warp; r < nc * (rows + 2); r += warps) {
+    const int c = r / (rows + 2), yy = y0 - 1 + r % (rows + 2);
+    const bool row_in = yy >= 0 && yy < H;
+    stage_row(sx + r * kTileS, x + (((size_t)n * C + c0 + c) * H + (row_in ? yy : 0)) * W, row_in, x0, W, wide);
+  }
+}
+// ReLU mask of staged gradients: zero where the staged output `sa` is not positive.
+__device__ __forceinline__ void mask_staged(float* sx, const float* sa, int nc, int rows, bool wide) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int r = warp; r < nc * (rows + 2); r += warps) {
+    float* v = sx + r * kTileS;
+    const float* m = sa + r * kTileS;
+    if (wide) {
+      if (lane < kTileS / 4) {
+        float4 g = ((float4*)v)[lane];
+        const float4 q = ((const float4*)m)[lane];
+        if (!(q.x > 0.0f)) g.x = 0.0f;
+        if (!(q.y > 0.0f)) g.y = 0.0f;
+        if (!(q.z > 0.0f)) g.z = 0.0f;
+        if (!(q.w > 0.0f)) g.w = 0.0f;
+        ((float4*)v)[lane] = g;
+      }
+      continue;
+    }
 #pragma unroll
-    for (int k = 0; k < 9; k++) {
-      const int yy = py + k / 3 - 1, xx = px + k % 3 - 1;
-      const float v = (yy >= 0 && yy < H && xx >= 0 && xx < W) ? xc[(size_t)yy * W + xx] : 0.0f;
-      const float* wr = sw + (ci * 9 + k) * COUT;
-      if constexpr (COUT % 4 == 0) {
+    for (int k = 0; k < 3; k++) {
+      const int j = lane + 32 * k + kTile0 - 1;
+      if (lane + 32 * k < kTile + 2 && !(m[j] > 0.0f)) v[j] = 0.0f;
+    }
+  }
+}
+
+// ---- 3x3 convolution to 32 channels -------------------------------------------------
+// Forward (BWD false): y = act(conv(x) + b) from C input channels.  Input
+// gradient (BWD true): the same sum over the C output channels of the layer
+// with the taps reversed, of the gradient masked by the layer's ReLU output.
+// A warp owns 64 pixels of one row and all 32 channels: lane (pixel group
+// lane & 7, channel group lane >> 3) holds eight pixels (4 g .. 4 g + 3 and 32
+// further on, so that 16-byte reads do not conflict) times eight channels as
+// channel pairs on the packed multiply-add, which one pixel value and one
+// weight pair feed: per input channel and kernel row 288 multiply-adds for
+// four reads of pixels and six of weights, where one thread per pixel read
+// eight times as many weights and was bound by those reads.  Per output the
+// terms are added in the order channel, row, column, starting from the bias.
+// The next channels are copied while the current ones are summed (loading them
+// between two barriers took half the time).  4 images of 256 x 512, 32 to 32
+// channels: 195 us forward and 230 us backward; one thread per pixel took three
+// times that.  The packed multiply-adds keep their pipe 70 % busy; what is left
+// is the operand reads of three-operand forms and the pixel pairs' moves.
+constexpr int kWStride = 36;  // floats per (channel, tap) row of 32 weights: 16-byte multiple, off the bank period
+template <bool BWD>
+__global__ void __launch_bounds__(256, 2) k_conv32(const float* __restrict__ x, const float* __restrict__ a, int C,
+                                                   int H, int W, const float* __restrict__ w,
+                                                   const float* __restrict__ b, int relu, float* __restrict__ y) {
+  extern __shared__ float4 smem4[];
+  // channels staged at a time: with a mask half as many, and their ReLU outputs
+  constexpr int kStep = BWD ? kChunk / 2 : kChunk;
+  float* sw = (float*)smem4;               // [C * 9][kWStride]
+  float* sbuf = sw + C * 9 * kWStride;     // two times [kChunk][rows + 2][kTileS]
+  const int rows = blockDim.x >> 5, row_tiles = (H + rows - 1) / rows;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pg = lane & 7, cg = lane >> 3;
+  const int n = blockIdx.y / row_tiles, y0 = (blockIdx.y % row_tiles) * rows, x0 = blockIdx.x * kTile;
+  for (int i = threadIdx.x; i < kMaxC * C * 9; i += blockDim.x) {
+    int o, r;
+    if (BWD) {  // w [c][o][tap]
+      const int c = i / (kMaxC * 9), k = i % 9;
+      o = (i / 9) % kMaxC;
+      r = c * 9 + 8 - k;
+    } else {  // w [o][c][tap]
+      o = i / (C * 9);
+      r = i % (C * 9);
+    }
+    copy4(sw + r * kWStride + o, w + i, true);
+  }
+  float2 acc[8][4];
 #pragma unroll
-        for (int j = 0; j < COUT / 4; j++) {
-          const float4 q = ((const float4*)wr)[j];
-          acc[4 * j] = fmaf(v, q.x, acc[4 * j]);
-          acc[4 * j + 1] = fmaf(v, q.y, acc[4 * j + 1]);
-          acc[4 * j + 2] = fmaf(v, q.z, acc[4 * j + 2]);
-          acc[4 * j + 3] = fmaf(v, q.w, acc[4 * j + 3]);
+  for (int c = 0; c < 4; c++) {
+    const float2 b2 = BWD ? make_float2(0.0f, 0.0f) : make_float2(b[8 * cg + 2 * c], b[8 * cg + 2 * c + 1]);
+#pragma unroll
+    for (int p = 0; p < 8; p++) acc[p][c] = b2;
+  }
+  const bool wide = wide_rows(x, a, W);
+  const int buf = kChunk * (rows + 2) * kTileS, masked = kStep * (rows + 2) * kTileS;
+  auto stage = [&](int c0) {
+    float* to = sbuf + (c0 / kStep & 1) * buf;
+    const int nc = min(kStep, C - c0);
+    stage_rows(x, n, C, c0, nc, H, W, x0, y0, rows, wide, to);
+    if (BWD && a) stage_rows(a, n, C, c0, nc, H, W, x0, y0, rows, wide, to + masked);
+    copies_commit();
+  };
+  stage(0);
+  for (int c0 = 0; c0 < C; c0 += kStep) {
+    const int nc = min(kStep, C - c0);
+    float* sx = sbuf + (c0 / kStep & 1) * buf;
+    if (c0 + kStep < C) {
+      stage(c0 + kStep);
+      copies_wait<1>();
+    } else {
+      copies_wait<0>();
+    }
+    if (BWD && a) mask_staged(sx, sx + masked, nc, rows, wide);
+    __syncthreads();
+    for (int ci = 0; ci < nc; ci++) {
+#pragma unroll
+      for (int ky = 0; ky < 3; ky++) {
+        const float* row = sx + (ci * (rows + 2) + warp + ky) * kTileS + kTile0 + 4 * pg;
+        float v[2][6];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const float4 q = *(const float4*)(row + 32 * h);
+          v[h][0] = row[32 * h - 1];
+          v[h][1] = q.x; v[h][2] = q.y; v[h][3] = q.z; v[h][4] = q.w;
+          v[h][5] = row[32 * h + 4];
         }
-      } else {
 #pragma unroll
-        for (int co = 0; co < COUT; co++) acc[co] = fmaf(v, wr[co], acc[co]);
-      }
-    }
-  }
-  float* yn = y + (size_t)n * COUT * plane + (size_t)py * W + px;
+        for (int kx = 0; kx < 3; kx++) {
+          const float4* wr = (const float4*)(sw + ((c0 + ci) * 9 + ky * 3 + kx) * kWStride + 8 * cg);
+          const float4 wa = wr[0], wb = wr[1];
+          const float2 wp[4] = {make_float2(wa.x, wa.y), make_float2(wa.z, wa.w), make_float2(wb.x, wb.y),
+                                make_float2(wb.z, wb.w)};
 #pragma unroll
-  for (int co = 0; co < COUT; co++) yn[co * plane] = relu ? fmaxf(acc[co], 0.0f) : acc[co];
-}
-
-// ---- backward, input gradient: one thread per input pixel, all 32 input channels --
-// gx[n, ci, y, x] = sum_co sum_k g[n, co, y + 1 - ky, x + 1 - kx] * w[co, ci, ky, kx],
-// with g = ga * (a > 0) when the layer has a ReLU (a != null).
-__global__ void __launch_bounds__(kRow) k_conv_bwd_data(const float* __restrict__ ga, const float* __restrict__ a,
-                                                        int COUT, int H, int W, const float* __restrict__ w,
-                                                        float* __restrict__ gx) {
-  constexpr int CIN = kMaxC;
-  extern __shared__ float4 sw4[];
-  float* sw = (float*)sw4;  // [COUT * 9][CIN]
-  for (int i = threadIdx.x; i < COUT * 9 * CIN; i += blockDim.x) {
-    const int ci = i % CIN, r = i / CIN, co = r / 9, k = r % 9;
-    sw[i] = w[(co * CIN + ci) * 9 + k];
-  }
-  __syncthreads();
-  const int px = blockIdx.x * kRow + threadIdx.x;
-  const int n = blockIdx.y / H, py = blockIdx.y % H;
-  if (px >= W) return;
-  const size_t plane = (size_t)H * W;
-  float acc[CIN];
+          for (int p = 0; p < 8; p++) {
+            const float2 xv = dup(v[p >> 2][(p & 3) + kx]);
 #pragma unroll
-  for (int ci = 0; ci < CIN; ci++) acc[ci] = 0.0f;
-  for (int co = 0; co < COUT; co++) {
-    const size_t base = ((size_t)n * COUT + co) * plane;
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-      const int yy = py + 1 - k / 3, xx = px + 1 - k % 3;
-      float g = 0.0f;
-      if (yy >= 0 && yy < H && xx >= 0 && xx < W) {
-        const size_t o = base + (size_t)yy * W + xx;
-        g = ga[o];
-        if (a && !(a[o] > 0.0f)) g = 0.0f;
-      }
-      const float4* wr = (const float4*)(sw + (co * 9 + k) * CIN);
-#pragma unroll
-      for (int j = 0; j < CIN / 4; j++) {
-        const float4 q = wr[j];
-        acc[4 * j] = fmaf(g, q.x, acc[4 * j]);
-        acc[4 * j + 1] = fmaf(g, q.y, acc[4 * j + 1]);
-        acc[4 * j + 2] = fmaf(g, q.z, acc[4 * j + 2]);
-        acc[4 * j + 3] = fmaf(g, q.w, acc[4 * j + 3]);
-      }
-    }
-  }
-  float* out = gx + (size_t)n * CIN * plane + (size_t)py * W + px;
-#pragma unroll
-  for (int ci = 0; ci < CIN; ci++) out[ci * plane] = acc[ci];
-}
-
-// ---- backward, weight gradient --------------------------------------------------
-// Thread t owns output channel co = t / 8 and input channels 4 (t % 8) .. +3,
-// all nine taps: 36 accumulators.  Tiles of 64 pixels of one row are staged in
-// shared memory (g for all output channels, three input rows with a 1-pixel
-// border); blocks stride over tiles and leave per-block partial sums.
-__global__ void __launch_bounds__(256) k_conv_bwd_weight(const float* __restrict__ x, const float* __restrict__ ga,
-                                                         const float* __restrict__ a, int N, int CIN, int COUT, int H,
-                                                         int W, float* __restrict__ partial) {
-  __shared__ float G[kMaxC][kWTile];
-  __shared__ float X[kMaxC][3][kWTile + 2];
-  const int t = threadIdx.x;
-  const int co = t / 8, cg = (t % 8) * 4;
-  const bool active = co < COUT && cg < CIN;
-  float acc[4][9];
-#pragma unroll
-  for (int j = 0; j < 4; j++)
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[j][k] = 0.0f;
-  float accb = 0.0f;
-  const size_t plane = (size_t)H * W;
-  const int tiles_x = (W + kWTile - 1) / kWTile;
-  const long long tiles = (long long)N * H * tiles_x;
-  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const int tx = (int)(tile % tiles_x);
-    const long long rowi = tile / tiles_x;
-    const int n = (int)(rowi / H), py = (int)(rowi % H);
-    const int x0 = tx * kWTile;
-    __syncthreads();
-    for (int i = t; i < kMaxC * kWTile; i += 256) {
-      const int c = i / kWTile, p = i % kWTile, xx = x0 + p;
-      float g = 0.0f;
-      if (c < COUT && xx < W) {
-        const size_t o = ((size_t)n * COUT + c) * plane + (size_t)py * W + xx;
-        g = ga[o];
-        if (a && !(a[o] > 0.0f)) g = 0.0f;
-      }
-      G[c][p] = g;
-    }
-    for (int i = t; i < CIN * 3 * (kWTile + 2); i += 256) {
-      const int c = i / (3 * (kWTile + 2)), r = (i / (kWTile + 2)) % 3, p = i % (kWTile + 2);
-      const int yy = py + r - 1, xx = x0 + p - 1;
-      X[c][r][p] = (yy >= 0 && yy < H && xx >= 0 && xx < W) ? x[((size_t)n * CIN + c) * plane + (size_t)yy * W + xx]
-                                                            : 0.0f;
-    }
-    __syncthreads();
-    if (active) {
-      const int nj = min(4, CIN - cg);
-      for (int p = 0; p < kWTile; p++) {
-        const float g = G[co][p];
-        accb += g;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          if (j < nj) {
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-              const float* xr = &X[cg + j][r][p];
-              acc[j][r * 3 + 0] = fmaf(g, xr[0], acc[j][r * 3 + 0]);
-              acc[j][r * 3 + 1] = fmaf(g, xr[1], acc[j][r * 3 + 1]);
-              acc[j][r * 3 + 2] = fmaf(g, xr[2], acc[j][r * 3 + 2]);
-            }
+            for (int c = 0; c < 4; c++) acc[p][c] = __ffma2_rn(xv, wp[c], acc[p][c]);
           }
         }
       }
     }
+    __syncthreads();  // this buffer takes the channels after the next
   }
-  const int nw = COUT * CIN * 9;
-  float* part = partial + (size_t)blockIdx.x * (nw + COUT);
-  if (active) {
-    for (int j = 0; j < 4 && cg + j < CIN; j++)
+  const int py = y0 + warp;
+  if (py >= H) return;
+  const size_t plane = (size_t)H * W;
+  const bool wide_out = wide_rows(y, nullptr, W);
 #pragma unroll
-      for (int k = 0; k < 9; k++) part[(co * CIN + cg + j) * 9 + k] = acc[j][k];
-    if (cg == 0) part[nw + co] = accb;
+  for (int c = 0; c < 8; c++) {
+    float* out = y + ((size_t)n * kMaxC + 8 * cg + c) * plane + (size_t)py * W;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int px = x0 + 32 * h + 4 * pg;
+      float r[4];
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const float2 q = acc[4 * h + p][c >> 1];
+        r[p] = (c & 1) ? q.y : q.x;
+        if (!BWD && relu) r[p] = fmaxf(r[p], 0.0f);
+      }
+      if (wide_out && px < W) {
+        *(float4*)(out + px) = make_float4(r[0], r[1], r[2], r[3]);
+      } else {
+#pragma unroll
+        for (int p = 0; p < 4; p++)
+          if (px + p < W) out[px + p] = r[p];
+      }
+    }
   }
 }
 
-// Sum the per-block partials [nblocks][nw + nb] in block order into the
-// weight gradient (first nw entries) and the bias gradient (last nb).
-__global__ void k_sum_partials(const float* __restrict__ partial, int nblocks, int nw, int nb, float* __restrict__ gw,
-                               float* __restrict__ gb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, n = nw + nb;
-  if (i >= n) return;
+// ---- forward to one channel: four pixels of a row per thread ------------------------
+// Bound by reading the input once: 16 threads cover a tile's row, 8 rows a
+// block, staged as above; 18 values serve 36 multiply-adds.
+__global__ void __launch_bounds__(kTile / 4 * 8) k_conv1(const float* __restrict__ x, int C, int H, int W,
+                                                         const float* __restrict__ w, const float* __restrict__ b,
+                                                         int relu, float* __restrict__ y) {
+  constexpr int kRows = 8;
+  __shared__ __align__(16) float sbuf[2][kChunk * (kRows + 2) * kTileS];
+  __shared__ float sw[kMaxC * 9];
+  const int row_tiles = (H + kRows - 1) / kRows, g = threadIdx.x % (kTile / 4), r = threadIdx.x / (kTile / 4);
+  const int n = blockIdx.y / row_tiles, y0 = (blockIdx.y % row_tiles) * kRows, x0 = blockIdx.x * kTile;
+  for (int i = threadIdx.x; i < C * 9; i += blockDim.x) sw[i] = w[i];
+  float acc[4] = {b[0], b[0], b[0], b[0]};
+  const bool wide = wide_rows(x, nullptr, W);
+  auto stage = [&](int c0) {
+    stage_rows(x, n, C, c0, min(kChunk, C - c0), H, W, x0, y0, kRows, wide, sbuf[c0 / kChunk & 1]);
+    copies_commit();
+  };
+  stage(0);
+  for (int c0 = 0; c0 < C; c0 += kChunk) {
+    const int nc = min(kChunk, C - c0);
+    const float* sx = sbuf[c0 / kChunk & 1];
+    if (c0 + kChunk < C) {
+      stage(c0 + kChunk);
+      copies_wait<1>();
+    } else {
+      copies_wait<0>();
+    }
+    __syncthreads();
+    for (int ci = 0; ci < nc; ci++)
+#pragma unroll
+      for (int ky = 0; ky < 3; ky++) {
+        const float* row = sx + (ci * (kRows + 2) + r + ky) * kTileS + kTile0 + 4 * g;
+        const float4 q = *(const float4*)row;
+        const float v[6] = {row[-1], q.x, q.y, q.z, q.w, row[4]};
+#pragma unroll
+        for (int kx = 0; kx < 3; kx++) {
+          const float wk = sw[(c0 + ci) * 9 + ky * 3 + kx];
+#pragma unroll
+          for (int p = 0; p < 4; p++) acc[p] = fmaf(v[p + kx], wk, acc[p]);
+        }
+      }
+    __syncthreads();
+  }
+  if (y0 + r >= H) return;
+  float* out = y + ((size_t)n * H + y0 + r) * W;
+#pragma unroll
+  for (int p = 0; p < 4; p++) {
+    const int px = x0 + 4 * g + p;
+    if (px < W) out[px] = relu ? fmaxf(acc[p], 0.0f) : acc[p];
+  }
+}
+
+// ---- backward, weight gradient --------------------------------------------------
+// gw[co][ci][k] = sum over pixels of g[co] x[ci] shifted by tap k, with
+// g = ga * (a > 0) when the layer has a ReLU.  Tiles of two rows of 64 pixels
+// are staged in shared memory (g of all output channels, four input rows with
+// a 1-pixel border).  A thread holds one input channel and four output
+// channels, all nine taps, as sums over the even and the odd pixels (the
+// packed multiply-add takes two neighbouring pixels of g and of x): per four
+// pixels 72 packed multiply-adds for four reads of g, the same for the whole
+// warp, and six of x.  Half of the 16 warps take each row of a tile; CINP lanes
+// hold the input channels, and the other lanes of a warp (CINP 4) or the other
+// warps (NCOG 1: at most four output channels) take other pixels.  Their sums
+// are added in a fixed order.  One block per multiprocessor strides over tiles
+// and copies the next tile while it sums the current one; blocks leave partial
+// sums.  4 images of 256 x 512, 32 to 32 channels: 300 us.
+constexpr int kWXChan = 4 * kTileS + 4;  // 292 floats a channel: 16-byte rows, 8-byte reads of 16 lanes conflict in pairs
+constexpr int kWThreads = 512;
+template <int CINP, int NCOG> struct WGeom {
+  static constexpr int kG = 4 * NCOG * 2 * kTile, kX = CINP * kWXChan;  // floats of one tile's g, x
+  static constexpr int kTileFloats = 2 * kG + kX;                       // g, the ReLU output, x
+  static constexpr int kRed = kWThreads / 32 * 36 * 32;                 // the warps' sums at the end
+  static constexpr size_t kSmem = (size_t)(2 * kTileFloats > kRed ? 2 * kTileFloats : kRed) * sizeof(float);
+};
+template <int CINP, int NCOG>
+__global__ void __launch_bounds__(kWThreads, 1)
+    k_conv_bwd_weight(const float* __restrict__ x, const float* __restrict__ ga, const float* __restrict__ a, int N,
+                      int CIN, int COUT, int H, int W, float* __restrict__ partial) {
+  using Geo = WGeom<CINP, NCOG>;
+  extern __shared__ float4 smem4[];
+  float* smem = (float*)smem4;
+  constexpr int kSplit = (32 / CINP) * (8 / NCOG), kSpan = kTile / kSplit;  // pixels of a row per thread
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int ci = lane % CINP, rr = warp >> 3, cog = (warp & 7) % NCOG;
+  const int split = ((warp & 7) / NCOG) * (32 / CINP) + lane / CINP;
+  float2 acc[4][9];
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int k = 0; k < 9; k++) acc[j][k] = make_float2(0.0f, 0.0f);
+  float accb = 0.0f;
+  const size_t plane = (size_t)H * W;
+  const int tiles_x = (W + kTile - 1) / kTile, tiles_y = (H + 1) / 2;
+  const long long tiles = (long long)N * tiles_y * tiles_x;
+  const bool wide = wide_rows(ga, a, W) && wide_rows(x, nullptr, W);
+  auto stage = [&](long long tile, float* G) {
+    float* A = G + Geo::kG;
+    float* X = A + Geo::kG;
+    const int x0 = (int)(tile % tiles_x) * kTile;
+    const long long rowi = tile / tiles_x;
+    const int n = (int)(rowi / tiles_y), y0 = (int)(rowi % tiles_y) * 2;
+    if (wide) {
+      for (int i = t; i < Geo::kG / 4; i += kWThreads) {
+        const int c = i / (2 * kTile / 4), yy = y0 + (i / (kTile / 4)) % 2, xx = x0 + 4 * (i % (kTile / 4));
+        const bool in = c < COUT && yy < H && xx < W;
+        const size_t o = in ? ((size_t)n * COUT + c) * plane + (size_t)yy * W + xx : 0;
+        copy16(G + 4 * i, ga + o, in);
+        if (a) copy16(A + 4 * i, a + o, in);
+      }
+    } else {
+      for (int i = t; i < Geo::kG; i += kWThreads) {
+        const int c = i / (2 * kTile), yy = y0 + (i / kTile) % 2, xx = x0 + i % kTile;
+        const bool in = c < COUT && yy < H && xx < W;
+        const size_t o = in ? ((size_t)n * COUT + c) * plane + (size_t)yy * W + xx : 0;
+        copy4(G + i, ga + o, in);
+        if (a) copy4(A + i, a + o, in);
+      }
+    }
+    for (int r = warp; r < CINP * 4; r += kWThreads / 32) {
+      const int c = r >> 2, yy = y0 + (r & 3) - 1;
+      const bool row_in = c < CIN && yy >= 0 && yy < H;
+      stage_row(X + c * kWXChan + (r & 3) * kTileS, x + (row_in ? ((size_t)n * CIN + c) * plane + (size_t)yy * W : 0),
+                row_in, x0, W, wide);
+    }
+    copies_commit();
+  };
+  int turn = 0;
+  if (blockIdx.x < tiles) stage(blockIdx.x, smem);
+  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x, turn ^= 1) {
+    float* G = smem + turn * Geo::kTileFloats;
+    const float* X = G + 2 * Geo::kG;
+    if (tile + gridDim.x < tiles) {
+      stage(tile + gridDim.x, smem + (turn ^ 1) * Geo::kTileFloats);
+      copies_wait<1>();
+    } else {
+      copies_wait<0>();
+    }
+    if (a) {  // (each thread masks its own copies)
+      if (wide) {
+        for (int i = t; i < Geo::kG / 4; i += kWThreads) {
+          float4 g = ((float4*)G)[i];
+          const float4 q = ((const float4*)(G + Geo::kG))[i];
+          if (!(q.x > 0.0f)) g.x = 0.0f;
+          if (!(q.y > 0.0f)) g.y = 0.0f;
+          if (!(q.z > 0.0f)) g.z = 0.0f;
+          if (!(q.w > 0.0f)) g.w = 0.0f;
+          ((float4*)G)[i] = g;
+        }
+      } else {
+        for (int i = t; i < Geo::kG; i += kWThreads)
+          if (!(G[Geo::kG + i] > 0.0f)) G[i] = 0.0f;
+      }
+    }
+    __syncthreads();
+    if (t < 4 * NCOG * 16) {  // bias: 16 threads per output channel
+#pragma unroll
+      for (int i = 0; i < 2 * kTile / 16; i++) accb += G[(t >> 4) * 2 * kTile + (t & 15) + 16 * i];
+    }
+    const float* gp = G + (4 * cog * 2 + rr) * kTile + split * kSpan;
+    const float* xp = X + ci * kWXChan + rr * kTileS + kTile0 + split * kSpan;
+    // pixels p, p + 1 of the three rows, and p - 1, p
+    float2 x2[3], left[3];
+#pragma unroll
+    for (int ky = 0; ky < 3; ky++) {
+      x2[ky] = *(const float2*)(xp + ky * kTileS);
+      left[ky] = make_float2(xp[ky * kTileS - 1], x2[ky].x);
+    }
+#pragma unroll 2
+    for (int p = 0; p < kSpan; p += 4) {
+      float4 g4[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) g4[j] = *(const float4*)(gp + j * 2 * kTile + p);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+#pragma unroll
+        for (int ky = 0; ky < 3; ky++) {
+          const float2 nx = *(const float2*)(xp + ky * kTileS + p + 2 * h + 2);
+          const float2 right = make_float2(x2[ky].y, nx.x);
+#pragma unroll
+          for (int kx = 0; kx < 3; kx++) {
+            const float2 xv = kx == 0 ? left[ky] : (kx == 1 ? x2[ky] : right);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              const float2 g = h ? make_float2(g4[j].z, g4[j].w) : make_float2(g4[j].x, g4[j].y);
+              acc[j][ky * 3 + kx] = __ffma2_rn(xv, g, acc[j][ky * 3 + kx]);
+            }
+          }
+          left[ky] = right;
+          x2[ky] = nx;
+        }
+      }
+    }
+    __syncthreads();  // this buffer takes the tile after the next
+  }
+  const int nw = COUT * CIN * 9;
+  float* part = partial + (size_t)blockIdx.x * (nw + COUT);
+  if (t < 4 * NCOG * 16) {  // (whole warps)
+    for (int d = 1; d < 16; d <<= 1) accb += __shfl_xor_sync(0xffffffffu, accb, d);
+    if ((t & 15) == 0 && (t >> 4) < COUT) part[nw + (t >> 4)] = accb;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      float s = acc[j][k].x + acc[j][k].y;
+#pragma unroll
+      for (int d = CINP; d < 32; d <<= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+      smem[(warp * 36 + j * 9 + k) * 32 + lane] = s;
+    }
+  __syncthreads();
+  // sum over the warps that share a group of output channels
+  for (int i = t; i < NCOG * 36 * CINP; i += kWThreads) {
+    const int c = i % CINP, e = (i / CINP) % 36, g = i / (CINP * 36), co = 4 * g + e / 9;
+    float s = 0.0f;
+#pragma unroll
+    for (int v = 0; v < kWThreads / 32; v += NCOG) s += smem[((v + g) * 36 + e) * 32 + c];
+    if (co < COUT && c < CIN) part[(co * CIN + c) * 9 + e % 9] = s;
+  }
+}
+
+// Sum the per-block partials [nblocks][nw + nb] into the weight gradient
+// (first nw entries) and the bias gradient (last nb): eight threads per entry
+// add a run of blocks each, and their sums are added in order.
+__global__ void __launch_bounds__(256) k_sum_partials(const float* __restrict__ partial, int nblocks, int nw, int nb,
+                                                      float* __restrict__ gw, float* __restrict__ gb) {
+  __shared__ float sh[8][32];
+  const int i = blockIdx.x * 32 + (threadIdx.x & 31), seg = threadIdx.x >> 5, n = nw + nb;
+  const int per = (nblocks + 7) / 8, b1 = min(nblocks, (seg + 1) * per);
   float s = 0.0f;
-  for (int bl = 0; bl < nblocks; bl++) s += partial[(size_t)bl * n + i];
+  if (i < n)
+    for (int bl = seg * per; bl < b1; bl++) s += partial[(size_t)bl * n + i];
+  sh[seg][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (seg != 0 || i >= n) return;
+#pragma unroll
+  for (int k = 1; k < 8; k++) s += sh[k][threadIdx.x];
   if (i < nw) gw[i] = s;
   else gb[i - nw] = s;
 }
@@ -256,11 +522,12 @@ __global__ void __launch_bounds__(256) k_closure_loss(const float* __restrict__ 
   if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
 }
 
+// One warp: each lane adds every 32nd partial, then the lanes in a fixed tree.
 __global__ void k_sum_double(const double* __restrict__ partial, int n, double scale, double* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
   double s = 0.0;
-  for (int i = 0; i < n; i++) s += partial[i];
-  *out = s * scale;
+  for (int i = threadIdx.x; i < n; i += 32) s += partial[i];
+  for (int d = 16; d > 0; d >>= 1) s += __shfl_down_sync(0xffffffffu, s, d);
+  if (threadIdx.x == 0) *out = s * scale;
 }
 
 // ---- Adam ------------------------------------------------------------------------------
@@ -366,6 +633,34 @@ __global__ void k_sample(const float* __restrict__ avg, const uint8_t* __restric
 
 bool bad_shape(int N, int C, int H, int W) { return N < 1 || C < 1 || H < 1 || W < 1 || (long long)N * H > 65535ll * 1024; }
 
+// Launch of k_conv32 over N images: eight rows a block where that fills the
+// multiprocessors twice, else fewer (a block's rows share its staged weights).
+int launch_conv32(bool bwd, const float* x, const float* a, int n, int C, int h, int w, const float* weight,
+                         const float* bias, int relu, float* y, cudaStream_t s) {
+  if ((long long)n * h > 65535) return cfail(LBM_ERR_CUDA, "convolution: n h = %lld above 65535", (long long)n * h);
+  const int tx = (w + kTile - 1) / kTile;
+  int rows = 8;
+  while (rows > 2 && (long long)tx * n * ((h + rows - 1) / rows) < 304) rows /= 2;
+  const size_t smem = ((size_t)C * 9 * kWStride + 2 * (size_t)kChunk * (rows + 2) * kTileS) * sizeof(float);
+  dim3 grid(tx, n * ((h + rows - 1) / rows));
+  auto kern = bwd ? k_conv32<true> : k_conv32<false>;
+  CCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<grid, 32 * rows, smem, s>>>(x, a, C, h, w, weight, bias, relu, y);
+  CCK(cudaGetLastError());
+  return LBM_OK;
+}
+
+template <int CINP, int NCOG>
+int launch_bwd_weight(const float* in, const float* grad_out, const float* out, int n, int cin, int cout, int h, int w,
+                      float* scratch, int blocks, cudaStream_t s) {
+  constexpr size_t smem = WGeom<CINP, NCOG>::kSmem;
+  auto kern = k_conv_bwd_weight<CINP, NCOG>;
+  CCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<blocks, kWThreads, smem, s>>>(in, grad_out, out, n, cin, cout, h, w, scratch);
+  CCK(cudaGetLastError());
+  return LBM_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -375,14 +670,11 @@ int lbm_cnn_conv_forward(const float* x, int n, int cin, int h, int w, const flo
   if (!x || !weight || !bias || !y) return cfail(LBM_ERR_ARG, "null pointer");
   if (bad_shape(n, cin, h, w) || cin > kMaxC || (cout != kMaxC && cout != 1))
     return cfail(LBM_ERR_ARG, "conv forward: shape n=%d cin=%d h=%d w=%d cout=%d", n, cin, h, w, cout);
-  dim3 grid((w + kRow - 1) / kRow, n * h);
-  const size_t smem = (size_t)cin * 9 * cout * sizeof(float);
-  if (cout == kMaxC) {
-    CCK(cudaFuncSetAttribute(k_conv_fwd<kMaxC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_conv_fwd<kMaxC><<<grid, kRow, smem, as_stream(stream)>>>(x, cin, h, w, weight, bias, relu, y);
-  } else {
-    k_conv_fwd<1><<<grid, kRow, smem, as_stream(stream)>>>(x, cin, h, w, weight, bias, relu, y);
-  }
+  if (cout == kMaxC)
+    return launch_conv32(false, x, nullptr, n, cin, h, w, weight, bias, relu, y, as_stream(stream));
+  if ((long long)n * h > 65535) return cfail(LBM_ERR_CUDA, "convolution: n h = %lld above 65535", (long long)n * h);
+  dim3 grid((w + kTile - 1) / kTile, n * ((h + 7) / 8));
+  k_conv1<<<grid, kTile / 4 * 8, 0, as_stream(stream)>>>(x, cin, h, w, weight, bias, relu, y);
   CCK(cudaGetLastError());
   return LBM_OK;
 }
@@ -392,12 +684,7 @@ int lbm_cnn_conv_backward_data(const float* grad_out, const float* out, int n, i
   if (!grad_out || !weight || !grad_in) return cfail(LBM_ERR_ARG, "null pointer");
   if (bad_shape(n, cin, h, w) || cin != kMaxC || cout < 1 || cout > kMaxC)
     return cfail(LBM_ERR_ARG, "conv backward data: shape n=%d cin=%d h=%d w=%d cout=%d", n, cin, h, w, cout);
-  dim3 grid((w + kRow - 1) / kRow, n * h);
-  const size_t smem = (size_t)cout * 9 * cin * sizeof(float);
-  CCK(cudaFuncSetAttribute(k_conv_bwd_data, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_conv_bwd_data<<<grid, kRow, smem, as_stream(stream)>>>(grad_out, out, cout, h, w, weight, grad_in);
-  CCK(cudaGetLastError());
-  return LBM_OK;
+  return launch_conv32(true, grad_out, out, n, cout, h, w, weight, nullptr, 0, grad_in, as_stream(stream));
 }
 
 int lbm_cnn_conv_backward_weight(const float* in, const float* grad_out, const float* out, int n, int cin, int h,
@@ -410,9 +697,13 @@ int lbm_cnn_conv_backward_weight(const float* in, const float* grad_out, const f
   if (scratch_bytes < (size_t)kWBlocks * per * sizeof(float))
     return cfail(LBM_ERR_ARG, "scratch needs %zu bytes", (size_t)kWBlocks * per * sizeof(float));
   cudaStream_t s = as_stream(stream);
-  k_conv_bwd_weight<<<kWBlocks, 256, 0, s>>>(in, grad_out, out, n, cin, cout, h, w, scratch);
-  CCK(cudaGetLastError());
-  k_sum_partials<<<(per + 255) / 256, 256, 0, s>>>(scratch, kWBlocks, nw, cout, grad_weight, grad_bias);
+  const long long tiles = (long long)n * ((h + 1) / 2) * ((w + kTile - 1) / kTile);
+  const int blocks = (int)(tiles < kWBlocks / 2 ? tiles : kWBlocks / 2);  // one per multiprocessor at most
+  const int rc = cout <= 4 ? launch_bwd_weight<32, 1>(in, grad_out, out, n, cin, cout, h, w, scratch, blocks, s)
+                 : cin <= 4 ? launch_bwd_weight<4, 8>(in, grad_out, out, n, cin, cout, h, w, scratch, blocks, s)
+                            : launch_bwd_weight<32, 8>(in, grad_out, out, n, cin, cout, h, w, scratch, blocks, s);
+  if (rc) return rc;
+  k_sum_partials<<<(per + 31) / 32, 256, 0, s>>>(scratch, blocks, nw, cout, grad_weight, grad_bias);
   CCK(cudaGetLastError());
   return LBM_OK;
 }

@@ -215,3 +215,48 @@ def test_gpu_closure_step_equals_plain_step_at_the_same_omega(lbm, torch_cuda, s
     got, fb = run(om0, nan)
     np.testing.assert_array_equal(got, ref_0)
     assert fb == int(((mask == 0)[:, 1:]).sum()) * steps
+
+
+@pytest.mark.parametrize("n,h,w", [(1, 1, 1), (1, 2, 63), (2, 9, 64), (1, 17, 65), (3, 8, 132), (4, 80, 256)])
+@pytest.mark.parametrize("cin,cout", [(32, 32), (4, 32), (32, 1), (5, 32), (9, 1)])
+def test_gpu_conv_tiles_and_channel_remainders(lbm, torch_cuda, n, h, w, cin, cout):
+    """Each layer kernel at the edges of its 64 x 8 (2) pixel tiles and 8- and
+    4-channel steps, with 16-byte aligned rows and without, against float64.
+    Sums of at most 9 * 32 (forward, data) or n h w (weights) products: errors
+    stay below 1e-5 of the largest magnitude."""
+    torch = torch_cuda
+    F = torch.nn.functional
+    lib = lbm.load_library()
+    gen = torch.Generator().manual_seed(1000 * h + w + cin)
+    x = torch.randn(n, cin, h, w, generator=gen)
+    wt = torch.randn(cout, cin, 3, 3, generator=gen)
+    b = torch.randn(cout, generator=gen)
+    g = torch.randn(n, cout, h, w, generator=gen)
+    x64, w64, b64 = (t.double().requires_grad_(True) for t in (x, wt, b))
+    y64 = torch.relu(F.conv2d(x64, w64, b64, padding=1))
+    y64.backward(g.double())
+    pad = 1 if h == 17 else 0  # rows that start off a 16-byte boundary
+
+    def dev(t):
+        flat = torch.zeros(t.numel() + pad, device="cuda")
+        flat[pad:].copy_(t.reshape(-1))
+        return flat[pad:]
+
+    def ptr(t):
+        return ctypes.c_void_p(t.data_ptr())
+
+    dx, dw, db, dg = dev(x), dev(wt), dev(b), dev(g)
+    y = dev(torch.zeros(n, cout, h, w))
+    assert lib.lbm_cnn_conv_forward(ptr(dx), n, cin, h, w, ptr(dw), ptr(db), cout, 1, ptr(y), None) == 0
+    close(y.cpu().view(n, cout, h, w).numpy(), y64.detach().numpy())
+    size = lib.lbm_cnn_weight_scratch_bytes(cin, cout)
+    scratch = torch.empty(size // 4, device="cuda")
+    gw, gb = torch.empty(wt.numel(), device="cuda"), torch.empty(cout, device="cuda")
+    assert lib.lbm_cnn_conv_backward_weight(ptr(dx), ptr(dg), ptr(y), n, cin, h, w, cout, ptr(gw), ptr(gb),
+                                            ptr(scratch), size, None) == 0
+    close(gw.cpu().view(wt.shape).numpy(), w64.grad.numpy(), atol=1e-6)
+    close(gb.cpu().numpy(), b64.grad.numpy(), atol=1e-6)
+    if cin == 32:
+        gx = dev(torch.zeros(n, cin, h, w))
+        assert lib.lbm_cnn_conv_backward_data(ptr(dg), ptr(y), n, cin, h, w, ptr(dw), cout, ptr(gx), None) == 0
+        close(gx.cpu().view(n, cin, h, w).numpy(), x64.grad.numpy(), atol=1e-6)
