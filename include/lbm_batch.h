@@ -5,9 +5,11 @@
  * LBM_EDGE_CHANNEL and the same storage: frozen equilibrium inlet at its own
  * u_in on column 0, zero-gradient outflow, periodic top/bottom, half-way
  * bounce-back from its own mask, its own omega.
- * One lbm_batch_step advances every domain by one step in ONE persistent
- * kernel launch over a table of (domain, 256-column strip, row band) tiles;
- * runs of 20 steps are replayed from a CUDA graph captured on first use.
+ * lbm_batch_step advances every domain together: one persistent kernel
+ * launch per step over a table of (domain, 256-column strip, row band) tiles,
+ * or, for batches of 400,000 cells or more unless a schedule was fixed by hand
+ * or the autotuner found otherwise, one launch per three steps; runs of 20 (18)
+ * steps are replayed from a CUDA graph captured on first use.
  * Results are bit-identical to advancing each domain through lbm_sim.
  *
  * Storage: LBM_STORE_F32, LBM_STORE_F16, LBM_STORE_BF16.  Every call is
@@ -75,7 +77,7 @@ int lbm_batch_conservation(lbm_batch* batch, double* out);
 int lbm_batch_set_rounding(lbm_batch* batch, int mode, uint32_t seed);
 int lbm_batch_get_rounding(const lbm_batch* batch, int* mode, uint32_t* seed);
 
-/* Fix the schedule by hand: variant 0..5 = (ring stages, cells per thread,
+/* Fix the schedule by hand, one step per launch: variant 0..5 = (ring stages, cells per thread,
  * strip columns) (5,1,256) (6,1,256) (5,2,256) (8,2,256) (6,2,512)
  * (4,2,512), the 512-column strips for f16 / bf16 only (f32 runs variants 4
  * and 5 with 256-column strips); dynamic 0 = tiles sorted longest first and dealt

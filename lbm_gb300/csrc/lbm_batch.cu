@@ -21,6 +21,7 @@
 
 #include "../../include/lbm_batch.h"
 #include "lbm_stage.cuh"
+#include "lbm_multi.cuh"
 
 using namespace lbm;
 
@@ -49,13 +50,16 @@ int bfail(int code, const char* fmt, ...) {
 constexpr long long kPad = 4096;  // elements of padding around every buffer (halo copies stay inside)
 constexpr int kBuckets = 3;       // domain-height buckets: <= 128, <= 256, taller
 constexpr int kBlock = 128;
+// Batches of at least this many cells start with three-step launches
+// (stochastic rounding: the second figure), as single lattices do.
+constexpr uint64_t kMultiCells = 400000, kMultiCellsSr = 1600000;
 
 int bucket_of(int ny) { return ny <= 128 ? 0 : (ny <= 256 ? 1 : 2); }
 
 struct DomainDev {
   Layout L;
   void* f[2];
-  void* rest;
+  void* rest[2];  // three-step launches read one and write the other
   uint32_t* mask;
   void* mom;  // rho, jx, jy planes
   float omega;
@@ -71,7 +75,7 @@ struct DomainDev {
 // A tile's step arguments from its domain's descriptor.
 template <class S, class C>
 __device__ void fill_args(StepArgs<S, C>& sa, const DomainDev& d, int src_i, int dst_i, int materialised,
-                          int write_moments, int rows, int* flag, const SrArgs& sr, int domain) {
+                          int write_moments, int rows, int* flag, const SrArgs& sr, int domain, int rest_i) {
   sa.L = d.L;
   sa.src = (const S*)d.f[src_i];
   sa.dst = (S*)d.f[dst_i];
@@ -79,7 +83,7 @@ __device__ void fill_args(StepArgs<S, C>& sa, const DomainDev& d, int src_i, int
     sa.srcp[p] = sa.src + (long long)p * d.L.ps;
     sa.dstp[p] = sa.dst + (long long)p * d.L.ps;
   }
-  sa.rest = (S*)d.rest;
+  sa.rest = (S*)d.rest[rest_i];
   sa.mask = d.mask;
   sa.omega = (C)d.omega;
   sa.ref = d.ref;
@@ -113,7 +117,7 @@ __device__ void fill_args(StepArgs<S, C>& sa, const DomainDev& d, int src_i, int
 template <class St, int NS, int CPT, int W, bool SR = false>
 __global__ void __launch_bounds__(stage_threads<CPT, W>(), W != kStageW ? 3 : (CPT == 1 ? 4 : 6))
     k_batch_step(const DomainDev* __restrict__ doms, const int4* __restrict__ tiles, int ntiles, int src_i, int dst_i,
-                 int materialised, int write_moments, int dynamic, int* counter, int* flag, SrArgs sr) {
+                 int materialised, int write_moments, int dynamic, int* counter, int* flag, SrArgs sr, int rest_i) {
   using S = typename St::S;
   using C = typename St::C;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -152,7 +156,7 @@ __global__ void __launch_bounds__(stage_threads<CPT, W>(), W != kStageW ? 3 : (C
         if (k >= 2 && !__all_sync(0xffffffffu, mbar_wait(smem_addr(&args_free[k & 1]), (uint32_t)(((k - 2) >> 1) & 1)))) {
           if (lane == 0) atomicOr(flag, 2);
         }
-        if (lane == 0) fill_args(A, doms[T.x], src_i, dst_i, materialised, write_moments, T.w - T.z, flag, sr, T.x);
+        if (lane == 0) fill_args(A, doms[T.x], src_i, dst_i, materialised, write_moments, T.w - T.z, flag, sr, T.x, rest_i);
         __syncwarp();
       }
       if (St::kDev && doms[T.x].ref.shift)
@@ -180,7 +184,7 @@ __global__ void __launch_bounds__(stage_threads<CPT, W>(), W != kStageW ? 3 : (C
     const int xb = T.y & 0x3FFFFFFF;
     const bool down = (T.y >> 30) != 0;
     if (threadIdx.x == 0)
-      fill_args(sa, doms[T.x], src_i, dst_i, materialised, write_moments, T.w - T.z, flag, sr, T.x);
+      fill_args(sa, doms[T.x], src_i, dst_i, materialised, write_moments, T.w - T.z, flag, sr, T.x, rest_i);
     __syncthreads();
     if (materialised) {
       const int x0 = xb + CPT * (int)threadIdx.x;
@@ -208,11 +212,32 @@ __global__ void __launch_bounds__(stage_threads<CPT, W>(), W != kStageW ? 3 : (C
   }
 }
 
+// Three steps over every tile: one CTA of one warp each, tile t = (domain,
+// first column, y0, y1).  The tile's arguments are set up in shared memory.
+template <class St, bool SR>
+__global__ void __launch_bounds__(32, kMultiOcc)
+    k_batch_multi(const DomainDev* __restrict__ doms, const CUtensorMap* __restrict__ maps,
+                  const int4* __restrict__ tiles, int src_i, int rest_i, int* flag, SrArgs sr, float one) {
+  using S = typename St::S;
+  using C = typename St::C;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t full[MultiGeom<S>::kStages];
+  __shared__ MultiArgs<S, C> m;
+  const int4 T = tiles[blockIdx.x];
+  if (threadIdx.x == 0) {
+    fill_args(m.a, doms[T.x], src_i, 1 - src_i, 0, 0, T.w - T.z, flag, sr, T.x, rest_i);
+    m.rest_out = (S*)doms[T.x].rest[1 - rest_i];
+    m.one = one;
+  }
+  __syncwarp();
+  multi_dispatch<St, SR>(m, maps + 2 * T.x + src_i, T.y, T.z, T.w, smem, full);
+}
+
 struct DomainHost {
   int nx, ny;
   float omega, u_in;
   Layout L;
-  size_t off_f[2], off_rest, off_mask, off_mom;  // byte offsets into the arena
+  size_t off_f[2], off_rest[2], off_mask, off_mom;  // byte offsets into the arena
   std::vector<uint8_t> mask;
 };
 
@@ -224,6 +249,7 @@ struct Config {
   int variant = 0;     // index into kVariants
   int dynamic = 0;     // 0: static longest-first round robin, 1: atomic tickets, 2: static through one ring
   int rows[kBuckets] = {32, 32, 32};
+  bool multi = false;  // three steps per launch where a call allows it (k_batch_multi)
 };
 
 // (ring depth, cells per thread)
@@ -244,6 +270,9 @@ struct lbm_batch {
   DomainDev* d_doms = nullptr;
   int4* d_tiles = nullptr;
   int ntiles = 0, tiles_cap = 0;
+  CUtensorMap* d_maps = nullptr;  // two per domain: the 8 planes of each buffer set
+  int4* d_mtiles = nullptr;       // tiles of the three-step launches
+  int nmtiles = 0, rest_i = 0;    // their number; the rest planes that hold the state
   int* d_counter = nullptr;  // one ticket counter per step of a captured graph
   int counters_cap = 0;
   int* d_flag = nullptr;
@@ -255,7 +284,7 @@ struct lbm_batch {
   uint64_t steps = 0, launches = 0, cells = 0;
   Config cfg;
   int grid = 0;  // persistent CTAs
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};  // kGraphSteps steps from buffer parity 0 / 1
+  cudaGraphExec_t graph[4] = {};  // a run of steps from each buffer and rest-plane parity
   std::string report;
   // stochastic rounding (16-bit storage): domain d uses seed sr_seed + d;
   // the step clock: clock_d holds the index of the first step not yet
@@ -338,6 +367,58 @@ int build_tiles(lbm_batch* b) {
   return LBM_OK;
 }
 
+template <class St> void* multi_kernel(bool sr) {
+  if constexpr (St::kDev) {
+    if (sr) return (void*)k_batch_multi<St, true>;
+  }
+  return (void*)k_batch_multi<St, false>;
+}
+size_t multi_smem(int storage) {
+  return storage == STORE_F32 ? (size_t)MultiGeom<float>::kStages * MultiGeom<float>::kBytes
+                              : (size_t)MultiGeom<__half>::kStages * MultiGeom<__half>::kBytes;
+}
+bool multi_default(const lbm_batch* b) { return b->cells >= (b->sr_on ? kMultiCellsSr : kMultiCells); }
+
+// Tensor maps and tiles of the three-step launches: bands of 8 to 24 rows, as
+// many as one wave of CTAs takes (the single lattice's rule over all domains).
+int build_multi(lbm_batch* b) {
+  std::vector<CUtensorMap> maps(2 * (size_t)b->count);
+  int sms = 0;
+  BCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
+  long long column_rows = 0;
+  for (const DomainHost& h : b->doms) column_rows += (long long)((h.nx + kMultiCols - 1) / kMultiCols) * h.ny;
+  const long long wave = (column_rows + kMultiOcc * sms - 1) / (kMultiOcc * sms);
+  const int want = (int)std::min(std::max(wave, 8ll), 24ll);
+  std::vector<int4> t;
+  for (int d = 0; d < b->count; d++) {
+    const DomainHost& h = b->doms[d];
+    for (int i = 0; i < 2; i++) {
+      void* f = b->arena + h.off_f[i];
+      if (!(b->storage == STORE_F32 ? encode_planes<float>(&maps[2 * d + i], h.L, f)
+                                    : encode_planes<__half>(&maps[2 * d + i], h.L, f)))
+        return bfail(LBM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    }
+    const int bands = (h.ny + want - 1) / want, rows = (h.ny + bands - 1) / bands;
+    for (int y0 = 0; y0 < h.ny; y0 += rows)
+      for (int xb = 0; xb < h.nx; xb += kMultiCols) t.push_back(make_int4(d, xb, y0, std::min(y0 + rows, h.ny)));
+  }
+  std::stable_sort(t.begin(), t.end(), [](const int4& x, const int4& y) { return x.w - x.z > y.w - y.z; });
+  b->nmtiles = (int)t.size();
+  BCK(cudaMalloc(&b->d_maps, maps.size() * sizeof(CUtensorMap)));
+  BCK(cudaMalloc(&b->d_mtiles, t.size() * sizeof(int4)));
+  BCK(cudaMemcpyAsync(b->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, b->stream));
+  BCK(cudaMemcpyAsync(b->d_mtiles, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
+  BCK(cudaStreamSynchronize(b->stream));
+  auto attr = [&](auto tag) -> int {
+    using St = decltype(tag);
+    for (int sr = 0; sr < 2; sr++)
+      BCK(cudaFuncSetAttribute(multi_kernel<St>(sr != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)multi_smem(b->storage)));
+    return LBM_OK;
+  };
+  return dispatch_st(b->storage, attr);
+}
+
 int configure(lbm_batch* b) {
   int rc = build_tiles(b);
   if (rc) return rc;
@@ -375,7 +456,7 @@ int launch_step(lbm_batch* b, bool write_moments, int* counter) {
   sr.t = b->clock_pending;
   sr.y0 = 0;
   void* args[] = {&b->d_doms, &b->d_tiles, &b->ntiles, (void*)&src, (void*)&dst, &mat, &wm, &dyn, &counter, &b->d_flag,
-                  &sr};
+                  &sr, &b->rest_i};
   auto go = [&](auto tag) -> int {
     using St = decltype(tag);
     BCK(cudaLaunchKernel(variant_kernel<St>(b->cfg.variant, b->sr_on != 0u), dim3(b->grid), dim3(W / CPT + 32), args,
@@ -389,6 +470,32 @@ int launch_step(lbm_batch* b, bool write_moments, int* counter) {
   b->materialised = false;
   b->steps++;
   if (b->sr_on) b->clock_pending++;
+  return LBM_OK;
+}
+
+// Three steps in one launch, without moments.
+int launch_steps3(lbm_batch* b) {
+  SrArgs sr;
+  sr.on = b->sr_on;
+  sr.seed = b->sr_seed;
+  sr.clock = b->sr_on ? b->clock_d : nullptr;
+  sr.t = b->clock_pending;
+  sr.y0 = 0;
+  float one = 1.0f;
+  void* args[] = {&b->d_doms, &b->d_maps, &b->d_mtiles, &b->cur, &b->rest_i, &b->d_flag, &sr, &one};
+  auto go = [&](auto tag) -> int {
+    using St = decltype(tag);
+    BCK(cudaLaunchKernel(multi_kernel<St>(b->sr_on != 0u), dim3(b->nmtiles), dim3(32), args, multi_smem(b->storage),
+                         b->stream));
+    return LBM_OK;
+  };
+  int rc = dispatch_st(b->storage, go);
+  if (rc) return rc;
+  b->launches++;
+  b->cur = 1 - b->cur;
+  b->rest_i ^= 1;
+  b->steps += kMultiSteps;
+  if (b->sr_on) b->clock_pending += kMultiSteps;
   return LBM_OK;
 }
 
@@ -412,7 +519,10 @@ int reset_clock(lbm_batch* b) {
   return LBM_OK;
 }
 
-constexpr int kGraphSteps = 20;  // steps per captured graph (even: the buffer parity repeats)
+constexpr int kGraphSteps = 20;       // steps per captured graph (even: the buffer parity repeats)
+constexpr int kGraphStepsMulti = 18;  // the same as six three-step launches (both parities repeat)
+int graph_steps(const lbm_batch* b) { return b->cfg.multi ? kGraphStepsMulti : kGraphSteps; }
+cudaGraphExec_t& graph_of(lbm_batch* b) { return b->graph[b->cur + 2 * b->rest_i]; }
 
 int ensure_counters(lbm_batch* b) {
   if (b->counters_cap >= kGraphSteps + 1) return LBM_OK;
@@ -421,9 +531,9 @@ int ensure_counters(lbm_batch* b) {
   return LBM_OK;
 }
 
-// Capture kGraphSteps steps starting from the current buffer parity.
+// Capture a run of graph_steps steps starting from the current parity.
 int capture_graph(lbm_batch* b) {
-  cudaGraphExec_t& out = b->graph[b->cur];
+  cudaGraphExec_t& out = graph_of(b);
   if (out) {
     cudaGraphExecDestroy(out);
     out = nullptr;
@@ -434,11 +544,14 @@ int capture_graph(lbm_batch* b) {
   if (rc) return rc;
   cudaGraph_t g;
   BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  for (int k = 0; k < kGraphSteps && !rc; k++) rc = launch_step(b, false, b->d_counter + 1 + k);
+  if (b->cfg.multi)
+    for (int k = 0; k < kGraphStepsMulti && !rc; k += kMultiSteps) rc = launch_steps3(b);
+  else
+    for (int k = 0; k < kGraphSteps && !rc; k++) rc = launch_step(b, false, b->d_counter + 1 + k);
   if (!rc) rc = advance_clock(b);  // recorded: every replay advances the clock
   b->clock_pending = 0;
   cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-  b->cur = cur0;  // capture recorded the launches without running them
+  b->cur = cur0;  // capture recorded the launches without running them (the rest planes end where they began)
   b->steps = steps0;
   b->launches = launches0;
   if (rc) return rc;
@@ -488,6 +601,8 @@ void release(lbm_batch* b) {
   cudaFree(b->arena);
   cudaFree(b->d_doms);
   cudaFree(b->d_tiles);
+  cudaFree(b->d_maps);
+  cudaFree(b->d_mtiles);
   cudaFree(b->d_counter);
   cudaFree(b->d_flag);
   cudaFree(b->clock_d);
@@ -546,7 +661,8 @@ int lbm_batch_create(uint32_t count, const uint32_t* nx, const uint32_t* ny, con
     h.L.ps = ((long long)h.L.pitch * h.ny + 127) / 128 * 128;
     h.off_f[0] = take(8 * (size_t)h.L.ps * b->es);
     h.off_f[1] = take(8 * (size_t)h.L.ps * b->es);
-    h.off_rest = take((size_t)h.L.ps * b->es);
+    h.off_rest[0] = take((size_t)h.L.ps * b->es);
+    h.off_rest[1] = take((size_t)h.L.ps * b->es);
     h.off_mask = take((size_t)h.L.mw * h.ny * 4);
     h.off_mom = take(3 * (size_t)h.L.ps * b->cs);
     h.mask.assign((size_t)h.nx * h.ny, 0);
@@ -574,7 +690,8 @@ int lbm_batch_create(uint32_t count, const uint32_t* nx, const uint32_t* ny, con
     dd[d].L = h.L;
     dd[d].f[0] = b->arena + h.off_f[0];
     dd[d].f[1] = b->arena + h.off_f[1];
-    dd[d].rest = b->arena + h.off_rest;
+    dd[d].rest[0] = b->arena + h.off_rest[0];
+    dd[d].rest[1] = b->arena + h.off_rest[1];
     dd[d].mask = (uint32_t*)(b->arena + h.off_mask);
     dd[d].mom = b->arena + h.off_mom;
     dd[d].omega = h.omega;
@@ -583,6 +700,8 @@ int lbm_batch_create(uint32_t count, const uint32_t* nx, const uint32_t* ny, con
   cudaMemcpyAsync(b->d_doms, dd.data(), count * sizeof(DomainDev), cudaMemcpyHostToDevice, b->stream);
   if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) return cleanup(LBM_ERR_CUDA, "setup", e);
   int rc = ensure_counters(b);
+  if (!rc) rc = build_multi(b);
+  b->cfg.multi = multi_default(b);
   if (!rc) rc = configure(b);
   if (!rc) rc = lbm_batch_init_equilibrium(b, 0.0f, 0);
   if (rc) {
@@ -636,7 +755,7 @@ int lbm_batch_init_equilibrium(lbm_batch* b, float noise_amp, uint64_t seed) {
       const DomainHost& h = b->doms[d];
       dim3 grid((h.nx + kBlock - 1) / kBlock, h.ny);
       k_init<St><<<grid, kBlock, 0, b->stream>>>(h.L, (S*)(b->arena + h.off_f[0]), (S*)(b->arena + h.off_f[1]),
-                                                  (S*)(b->arena + h.off_rest), 1.0f, h.u_in, 0.0f, noise_amp,
+                                                  (S*)(b->arena + h.off_rest[b->rest_i]), 1.0f, h.u_in, 0.0f, noise_amp,
                                                   seed + (uint64_t)d, 1, h.u_in, -1, -1,
                                                   domain_ref(h), nullptr);
     }
@@ -660,13 +779,19 @@ int lbm_batch_step(lbm_batch* b, uint32_t n) {
   for (uint32_t k = 0; k < n;) {
     const uint32_t left = n - k;
     const bool last = left == 1;
-    if (!b->materialised && !last && left > (uint32_t)kGraphSteps) {
-      if (!b->graph[b->cur] && (rc = capture_graph(b))) return rc;
+    const uint32_t run = (uint32_t)graph_steps(b);
+    if (!b->materialised && !last && left > run) {
+      if (!graph_of(b) && (rc = capture_graph(b))) return rc;
       if ((rc = advance_clock(b))) return rc;
-      BCK(cudaGraphLaunch(b->graph[b->cur], b->stream));
-      b->launches += kGraphSteps + (b->sr_on ? 1 : 0);
-      b->steps += kGraphSteps;  // kGraphSteps is even: the buffer parity is unchanged
-      k += kGraphSteps;
+      BCK(cudaGraphLaunch(graph_of(b), b->stream));
+      b->launches += (b->cfg.multi ? run / kMultiSteps : run) + (b->sr_on ? 1 : 0);
+      b->steps += run;  // an even number: the buffer parity is unchanged
+      k += run;
+      continue;
+    }
+    if (b->cfg.multi && !b->materialised && left > (uint32_t)kMultiSteps) {
+      if ((rc = launch_steps3(b))) return rc;
+      k += kMultiSteps;
       continue;
     }
     if ((rc = launch_step(b, last, b->d_counter))) return rc;
@@ -700,7 +825,7 @@ int lbm_batch_read_field(lbm_batch* b, uint32_t domain, int field, float* out) {
       using St = decltype(tag);
       using S = typename St::S;
       k_moments<St><<<grid, kBlock, 0, b->stream>>>(h.L, (const S*)(b->arena + h.off_f[b->cur]),
-                                                   (const S*)(b->arena + h.off_rest), mom, mom + h.L.ps,
+                                                   (const S*)(b->arena + h.off_rest[b->rest_i]), mom, mom + h.L.ps,
                                                    mom + 2 * h.L.ps, domain_ref(h));
       BCK(cudaGetLastError());
       return LBM_OK;
@@ -737,7 +862,7 @@ int lbm_batch_conservation(lbm_batch* b, double* out) {
         using St = decltype(tag);
         using S = typename St::S;
         k_moments<St><<<grid, kBlock, 0, b->stream>>>(h.L, (const S*)(b->arena + h.off_f[b->cur]),
-                                                     (const S*)(b->arena + h.off_rest), mom, mom + h.L.ps,
+                                                     (const S*)(b->arena + h.off_rest[b->rest_i]), mom, mom + h.L.ps,
                                                      mom + 2 * h.L.ps, domain_ref(h));
         BCK(cudaGetLastError());
         return LBM_OK;
@@ -769,7 +894,7 @@ int lbm_batch_read_populations(lbm_batch* b, uint32_t domain, float* out) {
     using St = decltype(tag);
     using S = typename St::S;
     k_read_pops<St, float><<<grid, kBlock, 0, b->stream>>>(h.L, (const S*)(b->arena + h.off_f[b->cur]),
-                                                           (const S*)(b->arena + h.off_rest), b->d_staging,
+                                                           (const S*)(b->arena + h.off_rest[b->rest_i]), b->d_staging,
                                                            domain_ref(h));
     BCK(cudaGetLastError());
     return LBM_OK;
@@ -793,6 +918,7 @@ int lbm_batch_set_rounding(lbm_batch* b, int mode, uint32_t seed) {
   b->sr_seed = b->sr_on ? seed : 0u;
   int rc = reset_clock(b);  // the clock counts on from the current step
   if (rc) return rc;
+  b->cfg.multi = b->cfg.multi && multi_default(b);
   return configure(b);  // the kernel, its occupancy and the captured graphs change
 }
 
@@ -809,6 +935,7 @@ int lbm_batch_set_schedule(lbm_batch* b, int variant, int dynamic, const int* ro
     return bfail(LBM_ERR_ARG, "bad schedule");
   b->cfg.variant = variant;
   b->cfg.dynamic = dynamic;
+  b->cfg.multi = false;
   if (rows_per_bucket)
     for (int i = 0; i < kBuckets; i++) b->cfg.rows[i] = std::max(1, rows_per_bucket[i]);
   return configure(b);
@@ -844,15 +971,15 @@ int lbm_batch_autotune(lbm_batch* b, uint32_t steps_per_trial, char* report, siz
   if (!b) return bfail(LBM_ERR_ARG, "null batch");
   const int T = (int)std::max(2u, steps_per_trial);
   std::string rep = "{\"trials\": [";
-  char buf[256];
+  char buf[512];
   bool first = true;
   auto trial = [&](const char* stage, float* best, Config* keep) -> int {
     float ms = 0.0f;
     int rc = time_config(b, T, &ms);
     if (rc) return rc;
     snprintf(buf, sizeof buf, "%s{\"stage\": \"%s\", \"variant\": %d, \"dynamic\": %d, \"rows\": [%d, %d, %d], "
-             "\"ms_per_step\": %.5f}", first ? "" : ", ", stage, b->cfg.variant, b->cfg.dynamic, b->cfg.rows[0],
-             b->cfg.rows[1], b->cfg.rows[2], ms / T);
+             "\"steps_per_launch\": %d, \"ms_per_step\": %.5f}", first ? "" : ", ", stage, b->cfg.variant, b->cfg.dynamic,
+             b->cfg.rows[0], b->cfg.rows[1], b->cfg.rows[2], b->cfg.multi ? kMultiSteps : 1, ms / T);
     rep += buf;
     first = false;
     if (ms < *best) {
@@ -862,6 +989,7 @@ int lbm_batch_autotune(lbm_batch* b, uint32_t steps_per_trial, char* report, siz
     return LBM_OK;
   };
   Config best_cfg = b->cfg;
+  best_cfg.multi = false;
   float best = 3.4e38f;
   // stage 1: ring depth x cells per thread x schedule
   const int variants = b->storage == STORE_F32 ? 2 : kNumVariants;
@@ -887,15 +1015,20 @@ int lbm_batch_autotune(lbm_batch* b, uint32_t steps_per_trial, char* report, siz
       if (rc) return rc;
     }
   }
+  // stage 3: three steps per launch, the schedule above for the other steps
   b->cfg = best_cfg;
-  int rc = configure(b);
+  b->cfg.multi = true;
+  int rc = trial("three_steps", &best, &best_cfg);
+  if (rc) return rc;
+  b->cfg = best_cfg;
+  rc = configure(b);
   if (rc) return rc;
   const int NS = kVariants[b->cfg.variant][0], CPT = kVariants[b->cfg.variant][1];
   snprintf(buf, sizeof buf, "], \"chosen\": {\"ring_stages\": %d, \"cells_per_thread\": %d, \"strip_columns\": %d, "
-           "\"schedule\": \"%s\", "
+           "\"schedule\": \"%s\", \"steps_per_launch\": %d, "
            "\"rows_per_band\": {\"ny<=128\": %d, \"ny<=256\": %d, \"ny>256\": %d}, \"ms_per_step\": %.5f, "
            "\"persistent_ctas\": %d, \"tiles\": %d}}",
-           NS, CPT, strip_of(b->cfg.variant, b->storage), b->cfg.dynamic == 1 ? "dynamic" : (b->cfg.dynamic == 2 ? "static_one_ring" : "static_longest_first"), b->cfg.rows[0], b->cfg.rows[1], b->cfg.rows[2],
+           NS, CPT, strip_of(b->cfg.variant, b->storage), b->cfg.dynamic == 1 ? "dynamic" : (b->cfg.dynamic == 2 ? "static_one_ring" : "static_longest_first"), b->cfg.multi ? kMultiSteps : 1, b->cfg.rows[0], b->cfg.rows[1], b->cfg.rows[2],
            best / T, b->grid, b->ntiles);
   rep += buf;
   b->report = rep;

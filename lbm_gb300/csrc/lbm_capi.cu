@@ -385,16 +385,10 @@ void release(lbm_sim* s) {
 
 // Tensor maps of both buffer sets for the three-step kernel's copies.
 bool encode_maps(lbm_sim* s) {
-  void* fn = nullptr;
-  cudaDriverEntryPointQueryResult found;
-  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
-      !fn)
-    return false;
-  for (int i = 0; i < 2; i++) {
-    const bool ok = s->es == 4 ? encode_planes<float>((EncodeTiledFn)fn, &s->planes[i], s->L, s->f[i])
-                               : encode_planes<__half>((EncodeTiledFn)fn, &s->planes[i], s->L, s->f[i]);
-    if (!ok) return false;
-  }
+  for (int i = 0; i < 2; i++)
+    if (!(s->es == 4 ? encode_planes<float>(&s->planes[i], s->L, s->f[i])
+                     : encode_planes<__half>(&s->planes[i], s->L, s->f[i])))
+      return false;
   return true;
 }
 
@@ -554,7 +548,6 @@ template <class St> int launch_multi(lbm_sim* s) {
   using G = MultiGeom<S>;
   MultiArgs<S, C> m;
   fill_step_args(s, m.a, 1 - s->cur);
-  m.planes = s->planes[s->cur];
   m.rest_out = (S*)s->rest_out;
   m.one = 1.0f;
   m.wcols = (s->L.nx + kMultiCols - 1) / kMultiCols;
@@ -578,7 +571,7 @@ template <class St> int launch_multi(lbm_sim* s) {
   // waves 143, 59 rows in one wave 153)
   const int bands = std::max(1, s->multi_occ * s->sms / m.wcols);
   m.a.rows = std::min(std::max((s->L.ny + bands - 1) / bands, 8), 24);
-  kern<<<m.wcols * ((s->L.ny + m.a.rows - 1) / m.a.rows), 32, smem, s->stream>>>(m);
+  kern<<<m.wcols * ((s->L.ny + m.a.rows - 1) / m.a.rows), 32, smem, s->stream>>>(s->planes[s->cur], m);
   CK_LAUNCH();
   return LBM_OK;
 }

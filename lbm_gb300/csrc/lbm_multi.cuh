@@ -231,7 +231,6 @@ __device__ __forceinline__ void tensor_g2s(uint32_t dst, const CUtensorMap* map,
 }
 
 template <class S, class C> struct MultiArgs {
-  CUtensorMap planes;  // the 8 planes of `src`
   StepArgs<S, C> a;
   S* rest_out;
   float one;  // 1 (see Ones)
@@ -241,8 +240,8 @@ template <class S, class C> struct MultiArgs {
 // One warp's tile: columns [xb, xb + 60) of rows [y0, y1).  EDGE: the tile
 // holds the inlet column, the outflow column or columns past it.
 template <class St, int KM, bool SR, bool EDGE>
-__device__ __forceinline__ void multi_tile(const MultiArgs<typename St::S, typename St::C>& m, int xb, int y0, int y1,
-                                           unsigned char* smem, uint64_t* full) {
+__device__ __forceinline__ void multi_tile(const MultiArgs<typename St::S, typename St::C>& m, const CUtensorMap* map,
+                                           int xb, int y0, int y1, unsigned char* smem, uint64_t* full) {
   using S = typename St::S;
   using Pr = Pair<St>;
   using P = typename Pr::P;
@@ -285,7 +284,7 @@ __device__ __forceinline__ void multi_tile(const MultiArgs<typename St::S, typen
     if (elect_one()) {
       const uint32_t st = smem_addr(smem + (size_t)s * G::kBytes), bar = smem_addr(&full[s]);
       mbar_arrive_expect_tx(bar, G::kCopied);
-      tensor_g2s(st, &m.planes, xs, rr, bar);
+      tensor_g2s(st, map, xs, rr, bar);
       bulk_g2s(st + 8 * G::kSegBytes, a.rest + ((long long)rr * L.pitch + xs), G::kSegBytes, bar);
       bulk_g2s(st + G::kMaskOff, a.mask + (long long)rr * L.mw + mw0, 32u, bar);
     }
@@ -481,43 +480,52 @@ __device__ __forceinline__ void multi_tile(const MultiArgs<typename St::S, typen
   if (!(rho_sum - rho_sum == 0.0f)) atomicOr(a.flag, 1);
 }
 
+// One warp's tile by the lattice's storage reference and the tile's edges
+// (the halo lanes advance the next two columns too, by their own rules).
+template <class St, bool SR>
+__device__ __forceinline__ void multi_dispatch(const MultiArgs<typename St::S, typename St::C>& m,
+                                               const CUtensorMap* map, int xb, int y0, int y1, unsigned char* smem,
+                                               uint64_t* full) {
+  const bool edge = xb == 0 || xb + kMultiCols + kMultiHalo >= m.a.L.nx;
+  if (St::kDev && m.a.ref.shift) {
+    if (edge) multi_tile<St, 1, SR, true>(m, map, xb, y0, y1, smem, full);
+    else multi_tile<St, 1, SR, false>(m, map, xb, y0, y1, smem, full);
+  } else {
+    if (edge) multi_tile<St, 0, SR, true>(m, map, xb, y0, y1, smem, full);
+    else multi_tile<St, 0, SR, false>(m, map, xb, y0, y1, smem, full);
+  }
+}
+
 template <class St, bool SR>
 __global__ void __launch_bounds__(32, kMultiOcc)
-    k_step_multi(const __grid_constant__ MultiArgs<typename St::S, typename St::C> m) {
+    k_step_multi(const __grid_constant__ CUtensorMap map,  // the 8 planes of `src`
+                 const __grid_constant__ MultiArgs<typename St::S, typename St::C> m) {
   using G = MultiGeom<typename St::S>;
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t full[G::kStages];
   const int band = blockIdx.x / m.wcols;
   const int xb = (blockIdx.x - band * m.wcols) * kMultiCols;
   const int y0 = band * m.a.rows, y1 = min(y0 + m.a.rows, m.a.row_end);
-  // (the halo lanes advance the next two columns too, by their own rules)
-  const bool edge = xb == 0 || xb + kMultiCols + kMultiHalo >= m.a.L.nx;
-  if constexpr (St::kDev) {
-    if (m.a.ref.shift) {
-      if (edge) multi_tile<St, 1, SR, true>(m, xb, y0, y1, smem, full);
-      else multi_tile<St, 1, SR, false>(m, xb, y0, y1, smem, full);
-    } else {
-      if (edge) multi_tile<St, 0, SR, true>(m, xb, y0, y1, smem, full);
-      else multi_tile<St, 0, SR, false>(m, xb, y0, y1, smem, full);
-    }
-  } else {
-    if (edge) multi_tile<St, 0, false, true>(m, xb, y0, y1, smem, full);
-    else multi_tile<St, 0, false, false>(m, xb, y0, y1, smem, full);
-  }
+  if (y0 >= y1) return;
+  multi_dispatch<St, SR>(m, &map, xb, y0, y1, smem, full);
 }
 
-// Host side: the map of a buffer set's 8 planes for k_step_multi's copies.
-// `encode` is the driver's cuTensorMapEncodeTiled.
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+// Host side: the tensor map of a buffer set's 8 planes, for the kernels' copies.
+template <class S> bool encode_planes(CUtensorMap* map, const Layout& L, void* planes) {
+  using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-template <class S> bool encode_planes(EncodeTiledFn encode, CUtensorMap* map, const Layout& L, void* planes) {
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+      !fn)
+    return false;
   const cuuint64_t dim[3] = {(cuuint64_t)L.pitch, (cuuint64_t)L.ny, 8};
   const cuuint64_t stride[2] = {(cuuint64_t)L.pitch * sizeof(S), (cuuint64_t)L.ps * sizeof(S)};
   const cuuint32_t box[3] = {(cuuint32_t)MultiGeom<S>::kSeg, 1, 8}, step[3] = {1, 1, 1};
-  return encode(map, sizeof(S) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, planes, dim,
-                stride, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return ((EncodeTiled)fn)(map, sizeof(S) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 3,
+                           planes, dim, stride, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                           CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace lbm

@@ -254,3 +254,47 @@ def test_gpu_sharded_batch_matches_the_whole(lbm, cuda_ok):
         lat.iterate(33)
         np.testing.assert_allclose(lat.conservation(), want[d], rtol=1e-12)
     whole.close()
+
+
+@pytest.mark.parametrize("storage,sr,scale", [(0, None, 1), (1, None, 1), (2, None, 1), (1, 77, 4)])
+def test_gpu_batch_three_step_launches_match_oracle_per_domain(lbm, cuda_ok, oracle_mod, storage, sr, scale):
+    """A batch large enough for three steps per launch (ragged domains around
+    its 60-column tiles, one of three rows): plain launches, captured runs, a
+    mask edit, fields and populations, every domain bit for bit."""
+    from lbm_gb300 import batch
+    P = oracle_mod
+    sizes = SIZES + [(60, 50), (61, 77), (121, 24), (700, 200)]
+    rng = np.random.default_rng(3)
+    nx = np.array([s[0] for s in sizes], np.uint32)
+    ny = np.array([s[1] * (scale if s[1] > 3 else 1) for s in sizes], np.uint32)
+    omega = (1.0 / rng.uniform(0.58, 0.8, len(sizes))).astype(np.float32)
+    u_in = rng.uniform(0.02, 0.07, len(sizes)).astype(np.float32)
+    masks = [(rng.random((int(y), int(x))) < 0.1).astype(np.uint8) for x, y in zip(nx, ny)]
+    with batch.Batch(nx, ny, omega, u_in, storage) as b:
+        assert b.info()[1] >= (400000 if sr is None else 1600000)
+        if sr is not None:
+            b.set_rounding(lbm.ROUND_STOCHASTIC, sr)
+        b.init_equilibrium(1e-2, 5)
+        orc = []
+        for d, m in enumerate(masks):
+            b.set_mask(d, m)
+            o = oracle_for(P, b, d, storage, m, 1e-2, 5)
+            if sr is not None:
+                o.set_rounding(1, sr + d)
+            orc.append(o)
+        done = 0
+        for n in (6, 45, 4):
+            b.step(n)
+            done += n
+            for o in orc:
+                o.step(n)
+            if n == 45:
+                m = masks[5].copy()
+                m[:, 100] = 1
+                m[::3, 100] = 0
+                b.set_mask(5, m)
+                orc[5].set_mask(m)
+        for d in range(b.count):
+            assert_domain(b, d, orc[d])
+        b.synchronize()
+        assert b.info()[2] == done
