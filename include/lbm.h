@@ -107,8 +107,8 @@ int lbm_get_stream(const lbm_sim* sim, void** cuda_stream);
  * for f32, 11 for f16 / bf16 (7 below 1024 columns), with rows_per_thread 8 for kernels 0 / 1 and a
  * band floor of 2 rows for the staged kernels; f64 storage always uses
  * kernel 0.  Until this is called, lbm_step takes three steps per launch
- * where it can (channel mode below f64, 400,000 cells or more, no closure);
- * the chosen kernel then takes every step by itself.  No counterpart in the reference, whose dispatch is fixed at
+ * where it can (channel mode below f64); the chosen kernel then takes every
+ * step by itself.  No counterpart in the reference, whose dispatch is fixed at
  * 256-wide 1-D workgroups (lbm.rs:102-106). */
 int lbm_set_tuning(lbm_sim* sim, int rows_per_thread, int kernel);
 

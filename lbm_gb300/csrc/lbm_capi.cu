@@ -13,6 +13,7 @@
 #include "lbm_kernels.cuh"
 #include "lbm_stage.cuh"
 #include "lbm_multi.cuh"
+#include "lbm_tile.cuh"
 #include "lbm_closure.cuh"
 #include "lbm_closure_tc.cuh"
 #include "lbm_render.cuh"
@@ -51,18 +52,28 @@ int fail(int code, const char* fmt, ...) {
 constexpr int kBlockX = 128;
 constexpr int kReduceBlocks = 608;  // 4 x 152 SMs
 constexpr long long kPadCells = 4096;
-// Channel lattices of at least this many cells take three steps per launch
-// (k_step_multi).  Us per step against the one-step kernels, graph replays of
-// 64-step calls, f32 / f16: 512 x 256 5.4 against 4.0 / 4.7 against 4.1;
-// 768 x 384 5.3 against 5.5 / 4.75 against 4.9; 1024 x 512 5.9 against 8.0 /
-// 5.3 against 6.7; 2048 x 1024 15.5 against 26.7 / 12.1 against 14.4;
-// 4096 x 2048 47.3 against 94.0 / 37.4 against 51.9.  Below it a warp's row
-// latency (about 1 us, three dependent collisions) is not hidden.
-constexpr uint64_t kMultiCells = 400000;
-// With stochastic rounding a level costs a third more, and three lattices
-// stepping at once (each filling the other's gaps) were 4 % slower at
-// 1531 x 769 and 17 % faster at 2048 x 1024.
-constexpr uint64_t kMultiCellsSr = 1600000;
+// Which kernel takes three steps in one launch (channel mode below f64), by
+// lattice size.  Two measurements decide: one lattice alone (us per step, 64-step
+// calls) and three lattices stepping at once, each filling the others' gaps.
+//   k_step_tile on small lattices.  Alone, f32 / f16, against the one-step
+//     kernels: 256 x 128 1.5 against 3.4 / 1.5 against 3.8; 512 x 256 2.1
+//     against 4.0 / 2.0 against 4.1; 768 x 384 4.0 against 5.5 / 3.7 against
+//     4.9.  Three at once: 512 x 256 1.35 / 1.31 times the speed; f16 at
+//     640 x 400 1.07, at 768 x 384 0.97.
+//   k_step_multi on larger ones.  Alone: 768 x 384 5.3 against 5.5 / 4.75
+//     against 4.9; 1024 x 512 5.9 against 8.0 / 5.3 against 6.7; 2048 x 1024
+//     15.5 against 26.7 / 12.1 against 14.4; 4096 x 2048 47 against 94 / 37
+//     against 52.  Three at once: f32 at 768 x 530 1.23 times the speed (the tile
+//     kernel 1.13), f16 at 1531 x 769 1.25.
+//   With stochastic rounding a step costs a third more: three at once were 4 %
+//     slower at 1531 x 769 and 17 % faster at 2048 x 1024; between the two
+//     kernels' ranges the one-step kernels stay.
+// The closure's steps run in k_step_tile: in f32 on any lattice, in 16-bit
+// storage on small ones.
+constexpr uint64_t kTileCells16 = 250000;     // k_step_tile below, 16-bit storage
+constexpr uint64_t kMultiCells32 = 400000;    // k_step_multi from here: f32 (k_step_tile below)
+constexpr uint64_t kMultiCells16 = 250000;    // 16-bit storage
+constexpr uint64_t kMultiCellsSr = 1600000;   // 16-bit storage with stochastic rounding
 
 size_t store_bytes(int storage) {
   switch (storage) {
@@ -529,16 +540,23 @@ template <class S, class C> void fill_step_args(const lbm_sim* s, StepArgs<S, C>
   a.sr.t = s->clock_pending;
 }
 
-// Whether a call may take three steps in one launch: the lattice's default
-// kernel in channel mode, a state past its first step (a materialised one is
-// collided in place), uniform omega, and the same words in column 0 of both
-// buffer sets (the levels of a launch pull the inlet from one of them).
-bool multi_ok(const lbm_sim* s) {
-  return s->rest_out && !s->tuned && !s->materialised && !s->closure_on && s->inlet_same &&
-         (!s->sr_on || (uint64_t)s->L.nx * s->L.ny >= kMultiCellsSr);
+// The kernel that takes three steps in one launch, if any (see kTileCells16).
+enum { THREE_NONE, THREE_TILE, THREE_ROWS };
+int three_kernel(const lbm_sim* s) {
+  const uint64_t cells = (uint64_t)s->L.nx * s->L.ny;
+  if (s->storage == STORE_F32) return s->closure_on || cells < kMultiCells32 ? THREE_TILE : THREE_ROWS;
+  if (cells < kTileCells16) return THREE_TILE;
+  if (s->closure_on) return THREE_NONE;
+  return cells >= (s->sr_on ? kMultiCellsSr : kMultiCells16) ? THREE_ROWS : THREE_NONE;
 }
-
-int multi_key(const lbm_sim* s) { return s->sr_on ? 1 : 0; }
+// Whether a call may take three steps in one launch: the lattice's default
+// kernel, a state past its first step (a materialised one is collided in
+// place), and the same words in column 0 of both buffer sets (the levels of a
+// launch pull the inlet from one of them).
+bool multi_ok(const lbm_sim* s) {
+  return s->rest_out && !s->tuned && !s->materialised && s->inlet_same && three_kernel(s) != THREE_NONE;
+}
+int multi_key(const lbm_sim* s) { return 4 * three_kernel(s) + (s->closure_on ? 2 : 0) + (s->sr_on ? 1 : 0); }
 
 // Three steps in one launch: reads buffer cur and `rest`, writes the other
 // buffer and `rest_out`; the caller updates the state.
@@ -551,28 +569,41 @@ template <class St> int launch_multi(lbm_sim* s) {
   m.rest_out = (S*)s->rest_out;
   m.one = 1.0f;
   m.wcols = (s->L.nx + kMultiCols - 1) / kMultiCols;
-  auto kern = k_step_multi<St, false>;
-  if constexpr (St::kDev) {
-    if (s->sr_on) kern = k_step_multi<St, true>;
+  const bool set = s->multi_variant != multi_key(s);
+  if (three_kernel(s) == THREE_ROWS) {
+    auto kern = k_step_multi<St, false>;
+    if constexpr (St::kDev) {
+      if (s->sr_on) kern = k_step_multi<St, true>;
+    }
+    const size_t smem = (size_t)G::kStages * G::kBytes;
+    if (set) {
+      CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      int occ = 0;
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32, smem));
+      if (occ < 1) return fail(LBM_ERR_CUDA, "three-step kernel does not fit on a multiprocessor");
+      s->multi_occ = occ;
+    }
+    // one wave of bands where that leaves 8 to 24 rows each: shorter bands
+    // repeat too many halo rows (2048 x 1024, f32: 16 rows 47 us a launch, 4 rows
+    // 58), taller ones wait for their last warp (4096 x 2048: 24 rows in 2.4
+    // waves 143, 59 rows in one wave 153)
+    const int bands = std::max(1, s->multi_occ * s->sms / m.wcols);
+    m.a.rows = std::min(std::max((s->L.ny + bands - 1) / bands, 8), 24);
+    kern<<<m.wcols * ((s->L.ny + m.a.rows - 1) / m.a.rows), 32, smem, s->stream>>>(s->planes[s->cur], m);
+  } else {
+    auto kern = s->closure_on ? k_step_tile<St, false, true> : k_step_tile<St, false, false>;
+    if constexpr (St::kDev) {
+      if (s->sr_on) kern = s->closure_on ? k_step_tile<St, true, true> : k_step_tile<St, true, false>;
+    }
+    if (set)
+      CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem<S>(kTileRows)));
+    // full tiles unless they leave multiprocessors idle
+    m.a.rows = m.wcols * ((s->L.ny + kTileRows - 1) / kTileRows) >= s->sms ? kTileRows : kTileRows / 2;
+    dim3 grid(m.wcols, (s->L.ny + m.a.rows - 1) / m.a.rows);
+    kern<<<grid, 32 * (m.a.rows + 2 * (kMultiSteps - 1)), tile_smem<S>(m.a.rows), s->stream>>>(m);
   }
-  const size_t smem = (size_t)G::kStages * G::kBytes;
-  const int variant = multi_key(s);
-  if (s->multi_variant != variant) {
-    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int occ = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32, smem));
-    if (occ < 1) return fail(LBM_ERR_CUDA, "three-step kernel does not fit on a multiprocessor");
-    s->multi_occ = occ;
-    s->multi_variant = variant;
-  }
-  // one wave of bands where that leaves 8 to 24 rows each: shorter bands
-  // repeat too many halo rows (2048 x 1024, f32: 16 rows 47 us a launch, 4 rows
-  // 58), taller ones wait for their last warp (4096 x 2048: 24 rows in 2.4
-  // waves 143, 59 rows in one wave 153)
-  const int bands = std::max(1, s->multi_occ * s->sms / m.wcols);
-  m.a.rows = std::min(std::max((s->L.ny + bands - 1) / bands, 8), 24);
-  kern<<<m.wcols * ((s->L.ny + m.a.rows - 1) / m.a.rows), 32, smem, s->stream>>>(s->planes[s->cur], m);
   CK_LAUNCH();
+  s->multi_variant = multi_key(s);
   return LBM_OK;
 }
 
@@ -656,7 +687,7 @@ int lbm_create(uint32_t nx, uint32_t ny, float omega, int edge_mode, int storage
   if ((rc = alloc_padded(&s->rest_base, &s->rest, (size_t)s->L.ps, s->es))) return rc;
   if ((rc = alloc_padded(&s->mask_base, (void**)&s->mask_d, (size_t)s->L.mw * ny, 4))) return rc;
   (void)plane;
-  if (edge_mode == EDGE_CHANNEL && storage != STORE_F64 && (uint64_t)nx * ny >= kMultiCells) {
+  if (edge_mode == EDGE_CHANNEL && storage != STORE_F64) {
     if ((rc = alloc_padded(&s->rest_out_base, &s->rest_out, (size_t)s->L.ps, s->es))) return rc;
     if (!encode_maps(s)) {
       release(s);

@@ -94,24 +94,10 @@ __device__ __forceinline__ void moments_f32_2(const float2 f[9], float2& rho, fl
   jy = add2(uy_c, k.sub(f[1], f[7]));
   rho = add2(add2(rho_c, add2(add2(add2(f[5], f[1]), f[7]), f[3])), f[4]);
 }
-template <bool NEAR>
-__device__ __forceinline__ void bgk_f32_2(float2 f[9], float2 rho, float2 jx, float2 jy, float w, const Ones& k,
-                                          bool divide, QuotRange& range, uint32_t solid) {
-  const float2 nb = mul2(rho, k.m), y = recip_rn2(rho, nb);
-  float2 ux = quot2(jx, nb, y), uy = quot2(jy, nb, y);
-  if (NEAR && divide) {
-    ux = make_float2(jx.x / rho.x, jx.y / rho.y);
-    uy = make_float2(jy.x / rho.x, jy.y / rho.y);
-  }
-  const float2 ux2 = mul2(ux, ux), uy2 = mul2(uy, uy);
-  const float2 u2 = k.add(ux2, uy2);
-  {  // (solid cells hold whatever words they were given and are never stored)
-    const bool sx = NEAR && (solid & 2u), sy = NEAR && (solid & 4u);
-    range.x |= sx ? 0u : __float_as_uint(rho.x) - 0x20000000u;
-    range.y |= sy ? 0u : __float_as_uint(rho.y) - 0x20000000u;
-    range.u2 = k.add(range.u2, NEAR ? make_float2(sx ? 0.0f : u2.x, sy ? 0.0f : u2.y) : u2);
-  }
-  const float2 w2 = dup2(w), c45 = dup2(4.5f);
+// Relaxation towards the equilibrium of velocity (ux, uy), u2 = |u|^2, at rates w2.
+__device__ __forceinline__ void relax_f32_2(float2 f[9], float2 rho, float2 ux, float2 uy, float2 ux2, float2 uy2,
+                                            float2 u2, float2 w2, const Ones& k) {
+  const float2 c45 = dup2(4.5f);
   const float2 ux3 = mul2(dup2(3.0f), ux), uy3 = mul2(dup2(3.0f), uy);
   const float2 uxuy2 = mul2(mul2(dup2(2.0f), ux), uy);
   const float2 u215 = mul2(dup2(1.5f), u2);
@@ -133,6 +119,45 @@ __device__ __forceinline__ void bgk_f32_2(float2 f[9], float2 rho, float2 jx, fl
   relax(3, r9, k.add(mx, sx));
   relax(1, r9, k.add(k.add(k.p, uy3), sy));
   relax(7, r9, k.add(k.sub(k.p, uy3), sy));
+}
+// NEAR: quotients by division on request, solid cells not in `range`.
+template <bool NEAR>
+__device__ __forceinline__ void bgk_f32_2(float2 f[9], float2 rho, float2 jx, float2 jy, float w, const Ones& k,
+                                          bool divide, QuotRange& range, uint32_t solid) {
+  const float2 nb = mul2(rho, k.m), y = recip_rn2(rho, nb);
+  float2 ux = quot2(jx, nb, y), uy = quot2(jy, nb, y);
+  if (NEAR && divide) {
+    ux = make_float2(jx.x / rho.x, jx.y / rho.y);
+    uy = make_float2(jy.x / rho.x, jy.y / rho.y);
+  }
+  const float2 ux2 = mul2(ux, ux), uy2 = mul2(uy, uy);
+  const float2 u2 = k.add(ux2, uy2);
+  {  // (solid cells hold whatever words they were given and are never stored)
+    const bool sx = NEAR && (solid & 2u), sy = NEAR && (solid & 4u);
+    range.x |= sx ? 0u : __float_as_uint(rho.x) - 0x20000000u;
+    range.y |= sy ? 0u : __float_as_uint(rho.y) - 0x20000000u;
+    range.u2 = k.add(range.u2, NEAR ? make_float2(sx ? 0.0f : u2.x, sy ? 0.0f : u2.y) : u2);
+  }
+  relax_f32_2(f, rho, ux, uy, ux2, uy2, u2, dup2(w), k);
+}
+// The same with the quotients checked at once and rates of two cells.
+__device__ __forceinline__ void bgk_f32_2_checked(float2 f[9], float2 rho, float2 jx, float2 jy, float2 w2,
+                                                  const Ones& k) {
+  const float2 nb = mul2(rho, k.m), y = recip_rn2(rho, nb);
+  float2 ux = quot2(jx, nb, y), uy = quot2(jy, nb, y);
+  float2 ux2 = mul2(ux, ux), uy2 = mul2(uy, uy), u2 = k.add(ux2, uy2);
+  QuotRange range;
+  range.x = __float_as_uint(rho.x) - 0x20000000u;
+  range.y = __float_as_uint(rho.y) - 0x20000000u;
+  range.u2 = u2;
+  if (!(range.ok_x() && range.ok_y())) {
+    ux = make_float2(jx.x / rho.x, jx.y / rho.y);
+    uy = make_float2(jy.x / rho.x, jy.y / rho.y);
+    ux2 = mul2(ux, ux);
+    uy2 = mul2(uy, uy);
+    u2 = k.add(ux2, uy2);
+  }
+  relax_f32_2(f, rho, ux, uy, ux2, uy2, u2, w2, k);
 }
 
 // Two adjacent columns of one direction as the levels keep them: a pair of
@@ -172,6 +197,39 @@ template <class St> struct Pair {  // 16-bit storage
     const float2 v = val(own);
     return word(make_float2(v.x + R.bb[q], v.y + R.bb[q]));
   }
+  __device__ static P make(S lo, S hi) {
+    S h[2] = {lo, hi};
+    uint32_t u;
+    memcpy(&u, h, 4);
+    return u;
+  }
+  template <int KM>
+  __device__ static void moments(const float2 f[9], float2& rho, float2& aux, float2& jx, float2& jy, const StoreRef& R,
+                                 const Ones&) {
+    St::template moments2<KM>(f, rho, aux, jx, jy, R);
+  }
+  // relaxation at a rate of its own per cell
+  __device__ static void relax(float2 f[9], float2 rho, float2 aux, float2 jx, float2 jy, float2 w, const StoreRef& R,
+                               const Ones&) {
+    float g[9];
+#pragma unroll
+    for (int q = 0; q < 9; q++) g[q] = f[q].x;
+    St::collide(g, rho.x, aux.x, jx.x, jy.x, w.x, R);
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+      f[q].x = g[q];
+      g[q] = f[q].y;
+    }
+    St::collide(g, rho.y, aux.y, jx.y, jy.y, w.y, R);
+#pragma unroll
+    for (int q = 0; q < 9; q++) f[q].y = g[q];
+  }
+  template <int KM>
+  __device__ static void collide_checked(float2 f[9], float2& rho, const typename St::Om& om, const StoreRef& R,
+                                         const Ones& k) {
+    QuotRange range;
+    collide<KM, false>(f, rho, om, R, k, false, range, 0u);
+  }
   template <int KM, bool NEAR>
   __device__ static void collide(float2 f[9], float2& rho, const typename St::Om& om, const StoreRef& R, const Ones&,
                                  bool, QuotRange&, uint32_t) {
@@ -195,6 +253,22 @@ template <> struct Pair<StF32> {
   __device__ static S half(P a, int j) { return j ? a.y : a.x; }
   __device__ static P take(P a, P b, int j) { return j ? make_float2(a.x, b.y) : make_float2(b.x, a.y); }
   template <int KM> __device__ static P bounce(P own, int, const StoreRef&) { return own; }
+  __device__ static P make(S lo, S hi) { return make_float2(lo, hi); }
+  template <int KM>
+  __device__ static void moments(const float2 f[9], float2& rho, float2&, float2& jx, float2& jy, const StoreRef&,
+                                 const Ones& k) {
+    moments_f32_2(f, rho, jx, jy, k);
+  }
+  __device__ static void relax(float2 f[9], float2 rho, float2, float2 jx, float2 jy, float2 w, const StoreRef&,
+                               const Ones& k) {
+    bgk_f32_2_checked(f, rho, jx, jy, w, k);
+  }
+  template <int KM>
+  __device__ static void collide_checked(float2 f[9], float2& rho, const float& om, const StoreRef&, const Ones& k) {
+    float2 jx, jy;
+    moments_f32_2(f, rho, jx, jy, k);
+    bgk_f32_2_checked(f, rho, jx, jy, dup2(om), k);
+  }
   template <int KM, bool NEAR>
   __device__ static void collide(float2 f[9], float2& rho, const float& om, const StoreRef&, const Ones& k, bool divide,
                                  QuotRange& range, uint32_t solid) {
