@@ -788,17 +788,21 @@ int lbm_set_barrier(lbm_sim* s, const uint32_t* pairs, size_t npairs) {
   int rc = materialise(s);
   if (!rc) rc = ensure_mask_host(s);
   if (rc) return rc;
+  // only the touched bits of the packed words change: packing whole rows again
+  // (350 rows of 1100 cells for a 300-point stroke) took 0.4 ms of a redraw
   const size_t n = s->mask_h.size();
   uint32_t ymin = UINT32_MAX, ymax = 0;
   for (size_t k = 0; k < npairs; k++) {
     size_t loc = pairs[2 * k];
     if (loc >= n) loc = n - 1;  // barrier_draw.wgsl:17 clamped store
-    s->mask_h[loc] = pairs[2 * k + 1] == 1u ? 1 : 0;
-    const uint32_t y = (uint32_t)(loc / s->L.nx);
+    const bool solid = pairs[2 * k + 1] == 1u;
+    const uint32_t y = (uint32_t)(loc / s->L.nx), x = (uint32_t)(loc % s->L.nx);
+    s->mask_h[loc] = solid ? 1 : 0;
+    uint32_t& word = s->words_h[(size_t)y * s->L.mw + (x >> 5)];
+    word = solid ? word | (1u << (x & 31)) : word & ~(1u << (x & 31));
     ymin = std::min(ymin, y);
     ymax = std::max(ymax, y);
   }
-  pack_words(s, ymin, ymax + 1);
   return upload_words(s, ymin, ymax + 1);
 }
 
@@ -1606,9 +1610,9 @@ int lbm_render(lbm_sim* s, int stat, int cmap, uint32_t width, uint32_t height, 
   if (!rgb && !rgba) return fail(LBM_ERR_ARG, "no output");
   const size_t px = (size_t)width * height;
   void* buf = nullptr;
-  CK(cudaMallocAsync(&buf, px * (12 + 4), s->stream));
-  float* d_rgb = (float*)buf;
-  uint8_t* d_rgba = (uint8_t*)buf + px * 12;
+  CK(cudaMallocAsync(&buf, px * ((rgb ? 12 : 0) + (rgba ? 4 : 0)), s->stream));
+  float* d_rgb = rgb ? (float*)buf : nullptr;
+  uint8_t* d_rgba = rgba ? (uint8_t*)buf + (rgb ? px * 12 : 0) : nullptr;
   int rc = frame(s, stat, cmap, width, height, d_rgb, d_rgba, srgb);
   if (!rc && rgb) rc = cudaMemcpyAsync(rgb, d_rgb, px * 12, cudaMemcpyDeviceToHost, s->stream) ? LBM_ERR_CUDA : 0;
   if (!rc && rgba) rc = cudaMemcpyAsync(rgba, d_rgba, px * 4, cudaMemcpyDeviceToHost, s->stream) ? LBM_ERR_CUDA : 0;
