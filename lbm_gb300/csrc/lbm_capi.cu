@@ -14,6 +14,7 @@
 #include "lbm_stage.cuh"
 #include "lbm_multi.cuh"
 #include "lbm_tile.cuh"
+#include "lbm_pair.cuh"
 #include "lbm_closure.cuh"
 #include "lbm_closure_tc.cuh"
 #include "lbm_render.cuh"
@@ -540,6 +541,12 @@ template <class S, class C> void fill_step_args(const lbm_sim* s, StepArgs<S, C>
   a.sr.t = s->clock_pending;
 }
 
+// Whether steps run in k_step_pair: reference mode below f64, a state past its
+// first step, no kernel chosen by lbm_set_tuning.
+bool pair_ok(const lbm_sim* s) {
+  return s->edge == EDGE_REF && s->storage != STORE_F64 && !s->tuned && !s->materialised;
+}
+
 // The kernel that takes three steps in one launch, if any (see kTileCells16).
 enum { THREE_NONE, THREE_TILE, THREE_ROWS };
 int three_kernel(const lbm_sim* s) {
@@ -988,10 +995,15 @@ int lbm_single_cell(lbm_sim* s, int dir) {
 // buffer cur and writing buffer `dst`; `last` writes the moments.  The
 // caller updates the state.
 static int launch_rows(lbm_sim* s, bool last, int row0, int row_end, int dst) {
-  const int rows = s->rows > 0 ? s->rows : 8;
   // f64 always runs the per-cell kernel: the pipelined and staged variants
-  // would spill its doubled register footprint.
-  const int variant = s->storage == STORE_F64 ? 0 : s->kernel;
+  // would spill its doubled register footprint.  One row per thread: the FP64
+  // pipe is the limit, and eight rows left it idle (1024 x 512 138 us a step
+  // against 115, 256 x 128 44 against 11).  The same kernel takes a small
+  // lattice's first step, which collides in place (256 x 128 6.1 us against 8.7
+  // in the staged kernel, 1100 x 700 13.0 against 14.9; 2048 x 1024 42 against 33).
+  const bool in_place = s->materialised && !s->tuned && (uint64_t)s->L.nx * s->L.ny < (1u << 20);
+  const int variant = s->storage == STORE_F64 || in_place ? 0 : s->kernel;
+  const int rows = s->rows > 0 ? s->rows : (variant == 0 ? 1 : 8);
   dim3 grid((s->L.nx + kBlockX - 1) / kBlockX, (row_end - row0 + rows - 1) / rows);
   auto launch = [&](auto tag) -> int {
     using St = decltype(tag);
@@ -1005,6 +1017,23 @@ static int launch_rows(lbm_sim* s, bool last, int row0, int row_end, int dst) {
     a.rho_out = last ? (C*)mom_plane(s, 0) : nullptr;
     a.jx_out = last ? (C*)mom_plane(s, 1) : nullptr;
     a.jy_out = last ? (C*)mom_plane(s, 2) : nullptr;
+    if constexpr (sizeof(S) <= 4) {
+      if (pair_ok(s)) {
+        PairArgs<S, C> m;
+        m.a = a;
+        m.one = 1.0f;
+        m.edge_ctas = (2 * (s->L.nx + s->L.ny - 2) + 32 * kPairWarps - 1) / (32 * kPairWarps);
+        m.cols = (s->L.nx + 63) / 64;
+        const int pairs = m.edge_ctas + m.cols * ((row_end - row0 + kPairWarps - 1) / kPairWarps);
+        auto kern = k_step_pair<St, false>;
+        if constexpr (St::kDev) {
+          if (s->sr_on) kern = k_step_pair<St, true>;
+        }
+        kern<<<pairs, 32 * kPairWarps, 0, s->stream>>>(m);
+        CK_LAUNCH();
+        return LBM_OK;
+      }
+    }
     if (variant >= 2) {
       return s->edge == EDGE_REF ? launch_staged_ns<St, EDGE_REF>(s, a) : launch_staged_ns<St, EDGE_CHANNEL>(s, a);
     } else if (variant == 1) {
@@ -1170,7 +1199,7 @@ int lbm_step(lbm_sim* s, uint32_t n) {
   if (s->stream != nullptr) CK(cudaStreamIsCapturing(s->stream, &capturing));
   auto steady = [&]() {
     return s->use_graphs && s->stream != nullptr && capturing == cudaStreamCaptureStatusNone && !s->materialised &&
-           (s->storage == STORE_F64 || s->kernel < 2 ||
+           (s->storage == STORE_F64 || s->kernel < 2 || pair_ok(s) ||
             s->staged_variant == staged_key(s->kernel, s->closure_on, s->sr_on != 0u)) &&
            (n <= (uint32_t)kMultiSteps || !multi_ok(s) || s->multi_variant == multi_key(s));
   };

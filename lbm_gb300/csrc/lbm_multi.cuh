@@ -225,6 +225,11 @@ template <class St> struct Pair {  // 16-bit storage
     for (int q = 0; q < 9; q++) f[q].y = g[q];
   }
   template <int KM>
+  __device__ static void relax_uniform(float2 f[9], float2 rho, float2 aux, float2 jx, float2 jy,
+                                       const typename St::Om& om, const StoreRef& R, const Ones&) {
+    St::template collide_u2<KM>(f, rho, aux, jx, jy, om, R);
+  }
+  template <int KM>
   __device__ static void collide_checked(float2 f[9], float2& rho, const typename St::Om& om, const StoreRef& R,
                                          const Ones& k) {
     QuotRange range;
@@ -262,6 +267,11 @@ template <> struct Pair<StF32> {
   __device__ static void relax(float2 f[9], float2 rho, float2, float2 jx, float2 jy, float2 w, const StoreRef&,
                                const Ones& k) {
     bgk_f32_2_checked(f, rho, jx, jy, w, k);
+  }
+  template <int KM>
+  __device__ static void relax_uniform(float2 f[9], float2 rho, float2, float2 jx, float2 jy, const float& om,
+                                       const StoreRef&, const Ones& k) {
+    bgk_f32_2_checked(f, rho, jx, jy, dup2(om), k);
   }
   template <int KM>
   __device__ static void collide_checked(float2 f[9], float2& rho, const float& om, const StoreRef&, const Ones& k) {
