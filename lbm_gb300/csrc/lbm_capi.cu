@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cstdarg>
 #include <cmath>
+#include <type_traits>
 
 #include "../../include/lbm.h"
 #include "lbm_kernels.cuh"
@@ -166,6 +167,10 @@ struct lbm_sim {
   cudaStream_t own_stream = nullptr, stream = nullptr;
   int cur = 0;               // buffer holding the latest state
   bool materialised = true;  // cur holds a pre-collision state
+  // the populations were read from the fused representation since the last
+  // step: a checkpoint, or a call on rows, made now sees the pre-collision
+  // state, as if the read had left it (a step leaves the same words either way)
+  bool pulled_read = false;
   bool moments_valid = false;
   uint64_t steps = 0, launches = 0;
   int rows = 0;    // rows per thread / band floor; 0: 8 for the per-cell kernels, 2 for the staged ones
@@ -321,6 +326,7 @@ int materialise(lbm_sim* s) {
   s->launches++;
   s->cur = dst;
   s->materialised = true;
+  s->pulled_read = false;
   return LBM_OK;
 }
 
@@ -353,6 +359,7 @@ int launch_init(lbm_sim* s, double rho, double ux, double uy, double amp, uint64
   s->launches++;
   s->cur = 0;
   s->materialised = true;
+  s->pulled_read = false;
   s->moments_valid = false;
   s->inlet_same = true;
   s->steps = 0;
@@ -1059,6 +1066,7 @@ static int launch_step(lbm_sim* s, bool last) {
   if (rc) return rc;
   s->cur = dst;
   s->materialised = false;
+  s->pulled_read = false;
   s->steps++;
   if (s->sr_on) s->clock_pending++;
   return LBM_OK;
@@ -1081,6 +1089,7 @@ static int launch_steps3(lbm_sim* s) {
   s->launches++;
   s->cur = 1 - s->cur;
   swap_rest(s);
+  s->pulled_read = false;
   s->steps += kMultiSteps;
   if (s->sr_on) s->clock_pending += kMultiSteps;
   return LBM_OK;
@@ -1181,6 +1190,7 @@ static int replay_steps(lbm_sim* s, StepRun* runs, uint32_t n, bool moments) {
   }
   if ((rc = advance_clock(s))) return rc;
   CK(cudaGraphLaunch(run.exec, s->stream));
+  s->pulled_read = false;
   s->steps += n;
   s->launches += run.launches;
   s->cur ^= (int)(n & 1u);
@@ -1229,6 +1239,10 @@ int lbm_step_rows(lbm_sim* s, uint32_t y0, uint32_t y1, int flags) {
   if (y0 >= y1 || y1 > (uint32_t)s->L.ny || (flags & ~(LBM_ROWS_COMPLETE | LBM_ROWS_MOMENTS)))
     return fail(LBM_ERR_ARG, "rows %u..%u of %d, flags 0x%x", y0, y1, s->L.ny, flags);
   if (s->pending < 0) {
+    if (s->pulled_read) {
+      int rc = materialise(s);
+      if (rc) return rc;
+    }
     s->pending = s->materialised ? s->cur : 1 - s->cur;
     s->pending_moments = true;
   }
@@ -1240,6 +1254,7 @@ int lbm_step_rows(lbm_sim* s, uint32_t y0, uint32_t y1, int flags) {
     s->cur = s->pending;
     s->pending = -1;
     s->materialised = false;
+    s->pulled_read = false;
     s->steps++;
     s->moments_valid = s->pending_moments;
     if (s->sr_on) s->clock_pending++;  // every row range of the step read the same index
@@ -1311,23 +1326,29 @@ int lbm_read_field_device(lbm_sim* s, int field, float* device_out) { return rea
 static int read_pops(lbm_sim* s, void* out, bool f64, bool device_out = false) {
   CHECK_SIM(s);
   if (!out) return fail(LBM_ERR_ARG, "out is null");
-  int rc = materialise(s);
-  if (rc) return rc;
   dim3 grid((s->L.nx + kBlockX - 1) / kBlockX, s->L.ny);
   void* mapped = device_out ? nullptr : mapped_host(out);
   void* dst = device_out ? out : (mapped ? mapped : (void*)s->staging_d);
-  auto launch = [&](auto tag) -> int {
+  auto launch_as = [&](auto tag, auto* o) -> int {
     using St = decltype(tag);
     using S = typename St::S;
-    if (f64)
-      k_read_pops<St, double><<<grid, kBlockX, 0, s->stream>>>(s->L, (const S*)s->f[s->cur], (const S*)s->rest,
-                                                                (double*)dst, store_ref(s));
+    using O = std::remove_pointer_t<decltype(o)>;
+    const StoreRef ref = store_ref(s);
+    const S *cur = (const S*)s->f[s->cur], *old = (const S*)s->f[1 - s->cur], *rest = (const S*)s->rest;
+    if (s->materialised)
+      k_read_pops<St, O><<<grid, kBlockX, 0, s->stream>>>(s->L, cur, rest, o, ref);
+    else if (s->edge == EDGE_REF)
+      k_read_pops_pulled<St, EDGE_REF, O><<<grid, kBlockX, 0, s->stream>>>(s->L, cur, old, rest, s->mask_d, o, ref);
     else
-      k_read_pops<St, float><<<grid, kBlockX, 0, s->stream>>>(s->L, (const S*)s->f[s->cur], (const S*)s->rest,
-                                                               (float*)dst, store_ref(s));
+      k_read_pops_pulled<St, EDGE_CHANNEL, O><<<grid, kBlockX, 0, s->stream>>>(s->L, cur, old, rest, s->mask_d, o, ref);
     CK_LAUNCH();
     return LBM_OK;
   };
+  auto launch = [&](auto tag) -> int {
+    return f64 ? launch_as(tag, (double*)dst) : launch_as(tag, (float*)dst);
+  };
+  s->pulled_read = !s->materialised;
+  int rc;
   rc = dispatch_storage(s->storage, launch);
   if (rc) return rc;
   s->launches++;
@@ -1381,6 +1402,7 @@ static int write_pops(lbm_sim* s, const void* in, bool f64) {
   if (rc) return rc;
   s->cur = 0;
   s->materialised = true;
+  s->pulled_read = false;
   s->moments_valid = false;
   s->inlet_same = true;
   s->steps = 0;
@@ -1735,6 +1757,7 @@ int lbm_checkpoint_save(lbm_sim* s, void* buf, size_t len) {
   const size_t need = sizeof(CkHeader) + ck_payload_bytes(s, closure);
   if (!buf || len < need) return fail(LBM_ERR_ARG, "checkpoint needs %zu bytes", need);
   int rc = ensure_mask_host(s);
+  if (!rc && s->pulled_read) rc = materialise(s);
   if (rc) return rc;
   const size_t cells = (size_t)s->L.nx * s->L.ny, e = s->es;
   CkHeader h{};
@@ -1866,6 +1889,7 @@ int lbm_checkpoint_load(lbm_sim* s, const void* buf, size_t len) {
   s->steps = h.steps;
   s->cur = (int)h.cur;
   s->materialised = h.materialised != 0;
+  s->pulled_read = false;
   s->moments_valid = false;
   s->inlet_same = true;  // column 0 of the two buffer sets
   for (size_t row = 0; row < 8 * (size_t)s->L.ny && s->inlet_same; row++)
@@ -1912,6 +1936,10 @@ static int rows_io(lbm_sim* s, uint32_t y, uint32_t nrows, uint32_t slot_mask, v
   // y >= ny || nrows > ny - y: no sum that could wrap in 32 bits
   if (nrows == 0 || y >= (uint32_t)s->L.ny || nrows > (uint32_t)s->L.ny - y || slot_mask == 0 || slot_mask > 0xFFu)
     return fail(LBM_ERR_ARG, "rows %u (+%u) of %d, slot mask 0x%x", y, nrows, s->L.ny, slot_mask);
+  if (s->pulled_read) {
+    int rc = materialise(s);
+    if (rc) return rc;
+  }
   const size_t e = s->es, row = (size_t)s->L.nx * e;
   const cudaMemcpyKind kind = read ? (on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost)
                                    : (on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);

@@ -498,6 +498,42 @@ __global__ void k_read_pops(Layout L, const typename St::S* f, const typename St
   }
 }
 
+// The same populations read from the fused representation (src: P_k, old: the
+// other buffer set): pulled with bounce-back, a bounced 16-bit word rounded for
+// its new direction, or the cell's own previous words where it is not streamed,
+// which is what k_materialise would leave behind, without writing it.  Bound by
+// memory: a read is one pass of 72 bytes a cell where materialising first was
+// two of 136, and the steps after it go on from the fused state (the first
+// step from a materialised one is a launch of its own, in place).
+template <class St, int EDGE, class O>
+__global__ void k_read_pops_pulled(Layout L, const typename St::S* __restrict__ src,
+                                   const typename St::S* __restrict__ old, const typename St::S* __restrict__ rest,
+                                   const uint32_t* __restrict__ mask, O* __restrict__ out, StoreRef ref) {
+  using S = typename St::S;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int y = blockIdx.y;
+  if (x >= L.nx) return;
+  const long long own = (long long)y * L.pitch + x;
+  const long long n = (long long)L.nx * L.ny, c = (long long)y * L.nx + x;
+  const bool still = mask_bit(mask, L.mw, x, y) || x == 0 || (EDGE == EDGE_REF && y == L.ny - 1);
+  const bool interior = x >= 1 && x <= L.nx - 2 && y >= 1 && y <= L.ny - 2;
+#pragma unroll
+  for (int q = 0; q < 9; q++) {
+    S v;
+    if (q == 4) {
+      v = rest[own];
+    } else if (still) {
+      v = old[(long long)slot(q) * L.ps + own];
+    } else {
+      int ux_ = x - cx(q), uy_ = y - cy(q);
+      if (!interior) upstream_edge<EDGE>(L, x, y, q, ux_, uy_);
+      v = mask_bit(mask, L.mw, ux_, uy_) ? St::store(St::bounce(src[(long long)slot(8 - q) * L.ps + own], q, ref), q)
+                                         : src[(long long)slot(q) * L.ps + (long long)uy_ * L.pitch + ux_];
+    }
+    out[q * n + c] = (O)St::f_of(v, q, ref);
+  }
+}
+
 // Bit-packs a dense nx-wide byte mask (nonzero = solid) into the pitched mask
 // words: one thread per word, bits past column nx-1 cleared.
 // The step clock of stochastic rounding: set it, or count launched steps in.

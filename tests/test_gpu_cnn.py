@@ -260,3 +260,41 @@ def test_gpu_conv_tiles_and_channel_remainders(lbm, torch_cuda, n, h, w, cin, co
         gx = dev(torch.zeros(n, cin, h, w))
         assert lib.lbm_cnn_conv_backward_data(ptr(dg), ptr(y), n, cin, h, w, ptr(dw), cout, ptr(gx), None) == 0
         close(gx.cpu().view(n, cin, h, w).numpy(), x64.grad.numpy(), atol=1e-6)
+
+
+@pytest.mark.parametrize("factor", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("h,w", [(3, 3), (4, 63), (5, 64), (6, 300)])
+def test_gpu_coarsened_blocks_by_whole_words_and_by_floats(lbm, torch_cuda, factor, h, w):
+    """Blocks read as 8- or 16-byte words against the same populations at an
+    address that only floats may be read from: the same bits; and against the
+    float64 oracle where every fluid cell is near rest (f32 sums of 9 F^2 terms
+    of order one: 1e-5 of the largest average)."""
+    torch = torch_cuda
+    from lbm_gb300 import closure
+    rng = np.random.default_rng(factor * 1000 + h * 10 + w)
+    hf, wf = h * factor, w * factor
+    W = np.array([1, 4, 1, 4, 16, 4, 1, 4, 1], np.float64)[:, None, None] / 36
+    pops = (W * (1 + 0.05 * rng.standard_normal((9, hf, wf)))).astype(np.float32)
+    solid = (rng.random((hf, wf)) < 0.3).astype(np.uint8)
+    s = torch.from_numpy(solid).cuda()
+    lib, stream = lbm.load_library(), None
+    out = []
+    for shift in (0, 1):
+        buf = torch.empty(9 * hf * wf + 4, dtype=torch.float32, device="cuda")
+        p = buf[shift:shift + 9 * hf * wf].view(9, hf, wf)
+        p.copy_(torch.from_numpy(pops))
+        feat = torch.empty((4, h, w), dtype=torch.float32, device="cuda")
+        coef = torch.empty((3, h, w), dtype=torch.float32, device="cuda")
+        scratch = torch.empty(6 * h * w, dtype=torch.float32, device="cuda")
+        solid_c = torch.empty((h, w), dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        closure.sample(lib, stream, p, s, factor, feat, coef, scratch, solid_c)
+        torch.cuda.synchronize()
+        out.append([t.cpu().numpy() for t in (feat, coef, scratch, solid_c)])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    want = C.coarsen(pops.astype(np.float64), solid, factor)
+    np.testing.assert_array_equal(out[0][3], want[-1])
+    avg = out[0][2].reshape(6, h, w)
+    rho = np.asarray(want[0])
+    np.testing.assert_allclose(avg[0], rho, rtol=0, atol=1e-5 * np.abs(rho).max())
