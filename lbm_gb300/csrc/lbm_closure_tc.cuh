@@ -2,7 +2,7 @@
 // network per 16 x 16 tile in shared memory, the three 32-channel layers as
 // implicit GEMMs issued with tcgen05.mma (BF16 operands from shared memory,
 // f32 accumulators in tensor memory) and the 1-channel output layer on the
-// CUDA cores (one output per thread).
+// CUDA cores.
 //
 // GEMM shapes per tile (M = window pixels, N = 32 output channels):
 //   layer 1  M = 22 rows x 24 (the feature window's pitch), 5 blocks of 128,
@@ -24,14 +24,15 @@
 // byte offset (next 8 K-values) is rows * 16 B and the stride byte offset
 // (next 8 rows) is 128 B.  Weights are [K / 8][N][8] likewise.
 //
-// Shared memory is 111 KB per CTA, so two CTAs share a multiprocessor and
+// Shared memory is 103 KB per CTA, so two CTAs share a multiprocessor and
 // one's epilogues run while the other's MMAs do.  Buffers are reused once
 // dead: the paired features and the layer-2 output share one region, the
 // layer-1 and layer-3 outputs another.  Every row a descriptor can reach
 // lies inside its region.
 //
-// One thread issues the MMAs and commits them to an mbarrier; every wait is
-// bounded (a timeout sets bit 2 of the error flag and the CTA stops waiting
+// A warp of its own issues the MMAs and commits each accumulator block to an
+// mbarrier, so the epilogue of a block runs while the next blocks' MMAs do;
+// every wait is bounded (a timeout sets bit 2 of the error flag and the CTA stops waiting
 // for the rest of its tiles).  Each CTA allocates 256 tensor-memory columns
 // (up to 5 accumulator blocks of 128 lanes x 32 f32) and frees them on every
 // path.
@@ -43,6 +44,8 @@
 namespace lbm {
 namespace tc {
 
+constexpr int kWorkers = 8, kWork = 32 * kWorkers;  // warps and threads of the features and epilogues
+constexpr int kThreads = kWork + 32;                // and the warp that issues the MMAs
 constexpr int kT = 16;                 // output tile
 constexpr int kW0 = kT + 8;            // feature window (24)
 constexpr int kW1 = kT + 6, kW2 = kT + 4, kW3 = kT + 2;  // layer output windows (22, 20, 18)
@@ -66,12 +69,12 @@ constexpr uint32_t kOffX1 = kOffP, kOffX3 = kOffP, kOffF = kOffQ, kOffX2 = kOffQ
 constexpr uint32_t kOffW1 = kOffQ + 4u * kRX2 * 16u;            // [6][32][8] bf16
 constexpr uint32_t kOffW2 = kOffW1 + 6u * 32u * 16u;            // [36][32][8] bf16
 constexpr uint32_t kOffW3 = kOffW2 + 36u * 32u * 16u;           // [36][32][8] bf16
-constexpr uint32_t kOffW4 = kOffW3 + 36u * 32u * 16u;           // [36][16][8] bf16: layer 4, output 0 of 16 (the
-                                                                // operand layout of an N = 16 GEMM; read on the CUDA cores)
-constexpr uint32_t kOffBias = kOffW4 + 36u * 16u * 16u;         // f32 b1 b2 b3 (32 each), b4
+constexpr uint32_t kOffW4 = kOffW3 + 36u * 32u * 16u;           // [9][32] f32 (rounded to bf16): layer 4
+constexpr uint32_t kOffBias = kOffW4 + 9u * 32u * 4u;           // f32 b1 b2 b3 (32 each), b4
 constexpr uint32_t kPackedBytes = kOffBias + 400u - kOffW1;     // 97 floats, padded to 16 B
-constexpr uint32_t kOffBar = kOffW1 + kPackedBytes;             // mbarrier (8 B), tensor-memory address (4 B)
-constexpr uint32_t kSmem = kOffBar + 16u;
+constexpr uint32_t kOffBar = kOffW1 + kPackedBytes;             // mbarriers: one per accumulator block, the parameters'
+constexpr uint32_t kOffTmem = kOffBar + 8u * (kB1 + 1);         // tensor-memory address (4 B)
+constexpr uint32_t kSmem = kOffTmem + 16u;
 static_assert(4u * kRX3 <= 4u * kRX1 && kRF <= 4 * kRX2, "buffer regions");
 static_assert(2u * (kSmem + 1024u) <= 233472u, "two CTAs per multiprocessor");
 static_assert(kPackedBytes % 16 == 0 && 97u * 4u <= 400u, "packed parameter block");
@@ -79,7 +82,8 @@ constexpr uint32_t kTmemCols = 256;    // power of two >= 32 x kB1
 
 // Host-side packing of the network parameters (cnn_layer_offset order, f32)
 // into the block copied verbatim into shared memory: BF16 weights in the
-// K-major operand layouts above; layer 4 and the biases as BF16-rounded f32.
+// K-major operand layouts above, those of layer 4 and the biases BF16-rounded
+// in f32.
 inline void pack_weights(const float* p, unsigned char* out) {
   auto bf = [](float v) { return __float2bfloat16_rn(v); };
   // layer 1: chunk kc = 2 ky + c holds taps kx = 2c (j < 4) and 2c + 1 (j >= 4)
@@ -100,13 +104,8 @@ inline void pack_weights(const float* p, unsigned char* out) {
           w[(kc * 32 + co) * 8 + j] = bf(p[cnn_layer_offset(l) + (co * 32 + ci) * 9 + tap]);
         }
   }
-  __nv_bfloat16* w4 = reinterpret_cast<__nv_bfloat16*>(out + kOffW4 - kOffW1);  // output 0 real, 1..15 zero
-  for (int kc = 0; kc < 36; kc++)
-    for (int co = 0; co < 16; co++)
-      for (int j = 0; j < 8; j++) {
-        const int tap = kc / 4, ci = (kc % 4) * 8 + j;
-        w4[(kc * 16 + co) * 8 + j] = bf(co == 0 ? p[cnn_layer_offset(3) + ci * 9 + tap] : 0.0f);
-      }
+  float* w4 = reinterpret_cast<float*>(out + kOffW4 - kOffW1);
+  for (int i = 0; i < 9 * 32; i++) w4[i] = __bfloat162float(bf(p[cnn_layer_offset(3) + (i % 32) * 9 + i / 32]));
   float* bias = reinterpret_cast<float*>(out + kOffBias - kOffW1);
   const int boff[4] = {cnn_layer_offset(1) - 32, cnn_layer_offset(2) - 32, cnn_layer_offset(3) - 32,
                        cnn_layer_offset(4) - 1};
@@ -163,12 +162,12 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
 // base descriptor plus a compile-time offset in its 14-bit address field
 // (all operands lie below 256 KB, so the field cannot carry).
 template <int BLOCKS, int TAPS, int KSTEPS, int A_ROWS, int PITCH, int N, uint32_t A_LBO = A_ROWS * 16u>
-__device__ __forceinline__ void issue_layer(uint32_t tmem, uint32_t a_base, uint32_t w_base) {
+__device__ __forceinline__ void issue_layer(uint32_t tmem, uint32_t a_base, uint32_t w_base, uint32_t bars) {
   constexpr uint32_t id = idesc(128, N);
   const uint64_t a0 = sdesc(a_base, A_LBO, 128u);
   const uint64_t b0 = sdesc(w_base, N * 16u, 128u);
 #pragma unroll
-  for (int mb = 0; mb < BLOCKS; mb++)
+  for (int mb = 0; mb < BLOCKS; mb++) {
 #pragma unroll
     for (int t = 0; t < TAPS; t++)
 #pragma unroll
@@ -180,6 +179,8 @@ __device__ __forceinline__ void issue_layer(uint32_t tmem, uint32_t a_base, uint
         const uint64_t b = b0 + (uint64_t)(kc * (uint32_t)N);
         mma(tmem + (uint32_t)(mb * 32), a, b, id, (t > 0 || s > 0) ? 1u : 0u);
       }
+    commit(bars + (uint32_t)(8 * mb));
+  }
 }
 
 // 32 consecutive f32 columns of this thread's tensor-memory lane.
@@ -202,34 +203,67 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 __device__ __forceinline__ void tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Store 32 channels of one pixel row into a [4][rows][8] bf16 buffer.
-__device__ __forceinline__ void store_row(unsigned char* buf, int rows, int row, const float (&v)[32]) {
+// acc + a * b, elementwise on two f32.
+__device__ __forceinline__ unsigned long long fma_pair(unsigned long long a, unsigned long long b,
+                                                       unsigned long long acc) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+  return acc;
+}
+__device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float pair_sum(unsigned long long v) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+  return lo + hi;
+}
+
+// A hidden layer's epilogue of one pixel row: bias, ReLU and bf16 of its 32
+// channels into row `row` of a [4][rows][8] buffer; zeros outside the lattice.
+__device__ __forceinline__ void store_row(unsigned char* buf, int rows, int row, const float (&v)[32],
+                                          const float* bias, bool inside) {
 #pragma unroll
   for (int c = 0; c < 4; c++) {
-    __nv_bfloat162 h[4];
+    uint32_t h[4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) h[j] = __floats2bfloat162_rn(v[8 * c + 2 * j], v[8 * c + 2 * j + 1]);
-    *reinterpret_cast<uint4*>(buf + ((size_t)c * rows + row) * 16) = *reinterpret_cast<uint4*>(h);
+    for (int j = 0; j < 4; j++) {
+      const int i = 8 * c + 2 * j;
+      const __nv_bfloat162 w = __floats2bfloat162_rn(fmaxf(v[i] + bias[i], 0.0f), fmaxf(v[i + 1] + bias[i + 1], 0.0f));
+      h[j] = inside ? *reinterpret_cast<const uint32_t*>(&w) : 0u;
+    }
+    *reinterpret_cast<uint4*>(buf + ((size_t)c * rows + row) * 16) = make_uint4(h[0], h[1], h[2], h[3]);
   }
 }
 
 }  // namespace tc
 
-// Persistent: grid = min(tiles, 2 x multiprocessors), 256 threads,
+// Persistent: grid = min(tiles, 2 x multiprocessors), tc::kThreads threads,
 // tc::kSmem dynamic shared memory; each CTA sets up tensor memory, its
-// mbarrier and the packed parameters once and then walks tiles blockIdx.x,
+// mbarriers and the packed parameters once and then walks tiles blockIdx.x,
 // + gridDim.x, ...
-__global__ void __launch_bounds__(256, 2)
+//
+// What bounds it: the MMAs, 48 cycles each (M 128, N 32, K 16: the A operand
+// from shared memory, whatever the order of the accumulators), 6800 cycles of
+// the 20,000 a tile takes beside another CTA's (15,000 alone), then the
+// epilogues.  512 x 256 (512 tiles in two turns) took 34.9 us with one
+// barrier a layer, the issuing thread an epilogue thread too, the parameters
+// copied by loads, window cells loaded one after the other and one output of
+// the last layer a thread; it takes 26.6 us, 2048 x 1024 283 against 398.
+// Warps 0 to 7 make the features, the epilogues and the
+// output layer; warp 8 issues the MMAs.
+__global__ void __launch_bounds__(tc::kThreads, 2)
     k_closure_infer_tc(Layout L, const float* __restrict__ rho, const float* __restrict__ jx,
                        const float* __restrict__ jy, const uint32_t* __restrict__ mask,
                        const unsigned char* __restrict__ wpack, float s_rho, float s_u, float dt_max,
                        __half2* __restrict__ record, int* __restrict__ flag) {
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char sm[];
-  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(sm + kOffBar + 8);
+  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(sm + kOffTmem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float* bias = reinterpret_cast<const float*>(sm + kOffBias);  // b1, b2, b3 (32 each), b4
-  const uint32_t bar = saddr(sm + kOffBar);
+  const uint32_t bars = saddr(sm + kOffBar), bar_w = bars + 8u * kB1;
   const uint32_t base = saddr(sm);
   const int tiles_x = (L.nx + kT - 1) / kT, tiles = tiles_x * ((L.ny + kT - 1) / kT);
 
@@ -238,27 +272,30 @@ __global__ void __launch_bounds__(256, 2)
                  "n"(kTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+  if (tid == 32 * kWorkers) {
+    for (int i = 0; i <= kB1; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8u * i));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  {  // packed parameters: one contiguous copy
-    const uint4* src = reinterpret_cast<const uint4*>(wpack);
-    uint4* dst = reinterpret_cast<uint4*>(sm + kOffW1);
-    for (int i = tid; i < (int)(kPackedBytes / 16); i += blockDim.x) dst[i] = src[i];
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // packed parameters: one bulk copy, waited for before the first layer
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_w), "n"(kPackedBytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     saddr(sm + kOffW1)),
+                 "l"(wpack), "n"(kPackedBytes), "r"(bar_w)
+                 : "memory");
   }
   tc_before();
   __syncthreads();
   tc_after();
   const uint32_t tmem = tmem_slot;
   const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
-  uint32_t phase = 0;
   bool ok = true;
 
-  // Waits for the MMAs thread 0 issued and committed (everyone).
-  auto wait_layer = [&]() {
-    if (ok && !bar_wait(bar, phase & 1u)) ok = false;
-    phase++;
+  // Waits for the MMAs of accumulator block mb of the layer in work: its
+  // barrier completes once per layer that has such a block.
+  uint32_t uses = 0;  // bit mb: parity of the uses of block mb's barrier so far
+  auto wait_block = [&](int mb) {
+    if (ok && !bar_wait(bars + 8u * mb, (uses >> mb) & 1u)) ok = false;
+    uses ^= 1u << mb;
     tc_after();
   };
   auto sync_async = [&]() {  // generic-proxy smem writes visible to the MMAs; TMEM reads done
@@ -268,35 +305,32 @@ __global__ void __launch_bounds__(256, 2)
     tc_after();
   };
 
-  // The features of a tile's 24 x 24 window: each thread owns window cells
+  // The features of a tile's 24 x 24 window: each worker owns window cells
   // tid, tid + 256, tid + 512.  The next tile's are loaded into registers
-  // while the current tile's layers run, so their latency is hidden.
-  constexpr int kFeatPer = (kW0 * kW0 + 255) / 256;
-  float4 fv[kFeatPer];
+  // while the current tile's layers run, so their latency is hidden: the mask
+  // word and the moments of a cell are loaded side by side and looked at when
+  // the features are stored.
+  constexpr int kFeatPer = (kW0 * kW0 + kWork - 1) / kWork;
+  float3 fv[kFeatPer];
+  uint32_t fm[kFeatPer], inside_m = 0;  // the mask word of the cell; bit k: the cell lies in the lattice
   auto load_feats = [&](int t) {
     const int fx0 = (t % tiles_x) * kT - 4, fy0 = (t / tiles_x) * kT - 4;
+    inside_m = 0;
 #pragma unroll
     for (int k = 0; k < kFeatPer; k++) {
-      const int i = tid + 256 * k;
-      float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (i < kW0 * kW0 && t < tiles) {
-        const int gx = fx0 + i % kW0, gy = fy0 + i / kW0;
-        if (gx >= 0 && gx < L.nx && gy >= 0 && gy < L.ny) {
-          const long long o = (long long)gy * L.pitch + gx;
-          if ((mask[(long long)gy * L.mw + (gx >> 5)] >> (gx & 31)) & 1u) {
-            f.w = 1.0f;
-          } else {  // raw moments now, scaled when stored
-            f.x = rho[o];
-            f.y = jx[o];
-            f.z = jy[o];
-            f.w = -1.0f;  // fluid marker
-          }
-        }
+      const int i = tid + kWork * k;
+      const int gx = fx0 + i % kW0, gy = fy0 + i / kW0;
+      if (i < kW0 * kW0 && t < tiles && gx >= 0 && gx < L.nx && gy >= 0 && gy < L.ny) {
+        const long long o = (long long)gy * L.pitch + gx;
+        inside_m |= 1u << k;
+        fm[k] = mask[(long long)gy * L.mw + (gx >> 5)];
+        fv[k] = make_float3(rho[o], jx[o], jy[o]);
       }
-      fv[k] = f;
     }
   };
-  load_feats(blockIdx.x);
+  if (warp < kWorkers) load_feats(blockIdx.x);
+
+  if (!bar_wait(bar_w, 0u)) ok = false;
 
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int tx0 = (tile % tiles_x) * kT, ty0 = (tile / tiles_x) * kT;
@@ -304,134 +338,162 @@ __global__ void __launch_bounds__(256, 2)
     // shares their region): window pixel i goes to the low half of row i and
     // the high half of row i - 1; rows from 575 on are zero beyond the window
     __syncthreads();
+    if (warp < kWorkers) {
 #pragma unroll
-    for (int k = 0; k < kFeatPer; k++) {
-      const int i = tid + 256 * k;
-      if (i >= kW0 * kW0) continue;
-      const float4 f = fv[k];
-      float4 o = make_float4(0.0f, 0.0f, 0.0f, f.w > 0.0f ? 1.0f : 0.0f);
-      if (f.w < 0.0f) {
-        o.x = (f.x - 1.0f) * s_rho;
-        o.y = f.y / f.x * s_u;
-        o.z = f.z / f.x * s_u;
+      for (int k = 0; k < kFeatPer; k++) {
+        const int i = tid + kWork * k;
+        if (i >= kW0 * kW0) continue;
+        float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if ((inside_m >> k) & 1u) {
+          if ((fm[k] >> ((tx0 - 4 + i % kW0) & 31)) & 1u) {
+            o.w = 1.0f;
+          } else {
+            const float3 f = fv[k];
+            o.x = (f.x - 1.0f) * s_rho;
+            o.y = f.y / f.x * s_u;
+            o.z = f.z / f.x * s_u;
+          }
+        }
+        __nv_bfloat162 h[2] = {__floats2bfloat162_rn(o.x, o.y), __floats2bfloat162_rn(o.z, o.w)};
+        const uint2 hv = *reinterpret_cast<uint2*>(h);
+        *reinterpret_cast<uint2*>(sm + kOffF + (size_t)i * 16) = hv;
+        if (i > 0) *reinterpret_cast<uint2*>(sm + kOffF + (size_t)(i - 1) * 16 + 8) = hv;
       }
-      __nv_bfloat162 h[2] = {__floats2bfloat162_rn(o.x, o.y), __floats2bfloat162_rn(o.z, o.w)};
-      const uint2 hv = *reinterpret_cast<uint2*>(h);
-      *reinterpret_cast<uint2*>(sm + kOffF + (size_t)i * 16) = hv;
-      if (i > 0) *reinterpret_cast<uint2*>(sm + kOffF + (size_t)(i - 1) * 16 + 8) = hv;
+      for (int i = kW0 * kW0 - 1 + tid; i < kRF; i += kWork) {
+        if (i == kW0 * kW0 - 1) *reinterpret_cast<uint2*>(sm + kOffF + (size_t)i * 16 + 8) = make_uint2(0u, 0u);
+        else *reinterpret_cast<uint4*>(sm + kOffF + (size_t)i * 16) = make_uint4(0u, 0u, 0u, 0u);
+      }
+      load_feats(tile + gridDim.x);  // in flight while this tile's layers run
     }
-    for (int i = kW0 * kW0 - 1 + tid; i < kRF; i += blockDim.x) {
-      if (i == kW0 * kW0 - 1) *reinterpret_cast<uint2*>(sm + kOffF + (size_t)i * 16 + 8) = make_uint2(0u, 0u);
-      else *reinterpret_cast<uint4*>(sm + kOffF + (size_t)i * 16) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    load_feats(tile + gridDim.x);  // in flight while this tile's layers run
     sync_async();
 
     // ---- layer 1 -> X1 (pitch 22) ---------------------------------------------------------
-    if (tid == 0) {
-      issue_layer<kB1, 3, 1, 0, kW0, 32, 32u>(tmem, base + kOffF, base + kOffW1);
-      commit(bar);
-    }
-    wait_layer();
-    for (int mb = warp >> 2; mb < kB1; mb += 2) {
+    if (tid == kWork) issue_layer<kB1, 3, 1, 0, kW0, 32, 32u>(tmem, base + kOffF, base + kOffW1, bars);
+    __syncwarp();
+    for (int mb = warp >> 2; mb < kB1 && warp < kWorkers; mb += 2) {
       float v[32];
+      wait_block(mb);
+      if (mb * 128 + 32 * (warp & 3) >= kM1) continue;  // (no row of the layer)
       tmem_ld32(tmem + lane_base + (uint32_t)(mb * 32), v);
       const int p = mb * 128 + 32 * (warp & 3) + lane;
       const int oy = p / kW0, ox = p % kW0;
       if (p < kM1 && ox < kW1) {
         const int gx = tx0 - 3 + ox, gy = ty0 - 3 + oy;
         const bool inside = gx >= 0 && gx < L.nx && gy >= 0 && gy < L.ny;
-#pragma unroll
-        for (int c = 0; c < 32; c++) v[c] = inside ? fmaxf(v[c] + bias[c], 0.0f) : 0.0f;
-        store_row(sm + kOffX1, kRX1, oy * kW1 + ox, v);
+        store_row(sm + kOffX1, kRX1, oy * kW1 + ox, v, bias, inside);
       }
     }
     // rows of X1 beyond the window: zero (read only by dropped outputs, but keep them finite)
-    for (int i = tid; i < 4 * (kRX1 - kW1 * kW1); i += blockDim.x) {
+    for (int i = tid; i < 4 * (kRX1 - kW1 * kW1) && warp < kWorkers; i += kWork) {
       const int c = i / (kRX1 - kW1 * kW1), r = kW1 * kW1 + i % (kRX1 - kW1 * kW1);
       *reinterpret_cast<uint4*>(sm + kOffX1 + ((size_t)c * kRX1 + r) * 16) = make_uint4(0u, 0u, 0u, 0u);
     }
     sync_async();
 
     // ---- layer 2 -> X2 (pitch 20, over the paired features) ---------------------------------
-    if (tid == 0) {
-      issue_layer<kB2, 9, 2, kRX1, kW1, 32>(tmem, base + kOffX1, base + kOffW2);
-      commit(bar);
-    }
-    wait_layer();
-    for (int mb = warp >> 2; mb < kB2; mb += 2) {
+    if (tid == kWork) issue_layer<kB2, 9, 2, kRX1, kW1, 32>(tmem, base + kOffX1, base + kOffW2, bars);
+    __syncwarp();
+    for (int mb = warp >> 2; mb < kB2 && warp < kWorkers; mb += 2) {
       float v[32];
+      wait_block(mb);
+      if (mb * 128 + 32 * (warp & 3) >= kM2) continue;  // (no row of the layer)
       tmem_ld32(tmem + lane_base + (uint32_t)(mb * 32), v);
       const int q = mb * 128 + 32 * (warp & 3) + lane;
       const int oy = q / kW1, ox = q % kW1;
       if (q < kM2 && ox < kW2) {
         const int gx = tx0 - 2 + ox, gy = ty0 - 2 + oy;
         const bool inside = gx >= 0 && gx < L.nx && gy >= 0 && gy < L.ny;
-#pragma unroll
-        for (int c = 0; c < 32; c++) v[c] = inside ? fmaxf(v[c] + bias[32 + c], 0.0f) : 0.0f;
-        store_row(sm + kOffX2, kRX2, oy * kW2 + ox, v);
+        store_row(sm + kOffX2, kRX2, oy * kW2 + ox, v, bias + 32, inside);
       }
     }
-    for (int i = tid; i < 4 * (kRX2 - kW2 * kW2); i += blockDim.x) {
+    for (int i = tid; i < 4 * (kRX2 - kW2 * kW2) && warp < kWorkers; i += kWork) {
       const int c = i / (kRX2 - kW2 * kW2), r = kW2 * kW2 + i % (kRX2 - kW2 * kW2);
       *reinterpret_cast<uint4*>(sm + kOffX2 + ((size_t)c * kRX2 + r) * 16) = make_uint4(0u, 0u, 0u, 0u);
     }
     sync_async();
 
-    // ---- layer 3 -> X3 (pitch 18, over X1) ----------------------------------------------------
-    if (tid == 0) {
-      issue_layer<kB3, 9, 2, kRX2, kW2, 32>(tmem, base + kOffX2, base + kOffW3);
-      commit(bar);
+    // the cell whose record this lane writes: its moments, in flight during layer 3
+    const int gx = tx0 + 8 * (warp & 1) + (lane & 7), gy = ty0 + 4 * (warp >> 1) + (lane >> 3);
+    const bool mine = warp < kWorkers && gx < L.nx && gy < L.ny;
+    const long long own = (long long)gy * L.pitch + gx;
+    float3 mom = make_float3(1.0f, 0.0f, 0.0f);
+    uint32_t own_word = 0;
+    if (mine) {
+      mom = make_float3(rho[own], jx[own], jy[own]);
+      own_word = mask[(long long)gy * L.mw + (gx >> 5)];
     }
-    wait_layer();
-    for (int mb = warp >> 2; mb < kB3; mb += 2) {
+
+    // ---- layer 3 -> X3 (pitch 18, over X1) ----------------------------------------------------
+    if (tid == kWork) issue_layer<kB3, 9, 2, kRX2, kW2, 32>(tmem, base + kOffX2, base + kOffW3, bars);
+    __syncwarp();
+    for (int mb = warp >> 2; mb < kB3 && warp < kWorkers; mb += 2) {
       float v[32];
+      wait_block(mb);
+      if (mb * 128 + 32 * (warp & 3) >= kM3) continue;  // (no row of the layer)
       tmem_ld32(tmem + lane_base + (uint32_t)(mb * 32), v);
       const int q = mb * 128 + 32 * (warp & 3) + lane;
       const int oy = q / kW2, ox = q % kW2;
       if (q < kM3 && ox < kW3) {
         const int gx = tx0 - 1 + ox, gy = ty0 - 1 + oy;
         const bool inside = gx >= 0 && gx < L.nx && gy >= 0 && gy < L.ny;
-#pragma unroll
-        for (int c = 0; c < 32; c++) v[c] = inside ? fmaxf(v[c] + bias[64 + c], 0.0f) : 0.0f;
-        store_row(sm + kOffX3, kRX3, oy * kW3 + ox, v);
+        store_row(sm + kOffX3, kRX3, oy * kW3 + ox, v, bias + 64, inside);
       }
     }
     sync_async();  // (the output layer reads only the 18 x 18 window: no tail rows to clear)
 
     // ---- layer 4 (32 -> 1) on the CUDA cores -> record -------------------------------------------
-    // One output per thread: 9 taps x 32 channels of X3 (pitch 18), four
-    // 16-byte rows per tap, against the layer's weights (output 0 of the
-    // packed [36][16][8] block, read by every thread at once: a broadcast).
-    // An N = 16 MMA for this one channel would stream 16 x more A operand
-    // from shared memory than the useful work needs.
-    {
-      const int oy = tid / kT, ox = tid % kT, gx = tx0 + ox, gy = ty0 + oy;
-      const unsigned char* x3 = sm + kOffX3;
-      const unsigned char* w4 = sm + kOffW4;
-      float z = bias[96];
+    // A warp takes 8 columns x 4 rows; a lane 8 of the 32 channels of the four
+    // outputs of its column, so that an activation (a 16-byte load) serves up
+    // to three outputs and a weight (a broadcast) four, two products per
+    // instruction; the channel groups are summed across lanes and lane (c, i)
+    // finishes row c of column i.  One output per thread took 1730 cycles a
+    // tile in shared-memory loads alone, this 720.  An N = 16 MMA for the one
+    // channel would stream 16 x more A operand than the useful work needs.
+    if (warp < kWorkers) {
+      const int c = lane >> 3, ox = 8 * (warp & 1) + (lane & 7), oy0 = 4 * (warp >> 1);
+      const unsigned char* x3 = sm + kOffX3 + ((size_t)c * kRX3 + oy0 * kW3 + ox) * 16;
+      const ulonglong2* w4 = reinterpret_cast<const ulonglong2*>(sm + kOffW4) + 2 * c;
+      unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
-      for (int t = 0; t < 9; t++) {
-        const int row = (oy + t / 3) * kW3 + ox + t % 3;
+      for (int kx = 0; kx < 3; kx++) {
+        unsigned long long w[3][4];
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-          const uint4 xv = *reinterpret_cast<const uint4*>(x3 + ((size_t)c * kRX3 + row) * 16);
-          const uint4 wv = *reinterpret_cast<const uint4*>(w4 + (size_t)((t * 4 + c) * 16) * 16);
-          const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w}, ws[4] = {wv.x, wv.y, wv.z, wv.w};
+        for (int ky = 0; ky < 3; ky++) {
+          const ulonglong2 w0 = w4[(ky * 3 + kx) * 8], w1 = w4[(ky * 3 + kx) * 8 + 1];
+          w[ky][0] = w0.x;
+          w[ky][1] = w0.y;
+          w[ky][2] = w1.x;
+          w[ky][3] = w1.y;
+        }
 #pragma unroll
-          for (int i = 0; i < 4; i++) {  // bf16 -> f32 is exact: the high 16 bits
-            z = __fmaf_rn(__uint_as_float(xs[i] << 16), __uint_as_float(ws[i] << 16), z);
-            z = __fmaf_rn(__uint_as_float(xs[i] & 0xFFFF0000u), __uint_as_float(ws[i] & 0xFFFF0000u), z);
+        for (int r = 0; r < 6; r++) {
+          const uint4 xv = *reinterpret_cast<const uint4*>(x3 + (size_t)(r * kW3 + kx) * 16);
+          const uint32_t xs[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+          for (int j = 0; j < 4; j++) {  // bf16 -> f32 is exact: the high 16 bits
+            const unsigned long long x =
+                pair_of(__uint_as_float(xs[j] << 16), __uint_as_float(xs[j] & 0xFFFF0000u));
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+              if (r - k >= 0 && r - k <= 2) acc[k] = fma_pair(x, w[r - k][j], acc[k]);
           }
         }
       }
-      if (gx < L.nx && gy < L.ny) {
-        const long long o = (long long)gy * L.pitch + gx;
+      float z = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        float p = pair_sum(acc[k]);
+        p += __shfl_xor_sync(0xffffffffu, p, 8);
+        p += __shfl_xor_sync(0xffffffffu, p, 16);
+        if (c == k) z = p;
+      }
+      z += bias[96];
+      if (mine) {
         const float dt = dt_max / (1.0f + expf(-z));
         // |u| of the cell (solid cells: 0), from its moments
-        const bool solid = (mask[(long long)gy * L.mw + (gx >> 5)] >> (gx & 31)) & 1u;
-        const float r = rho[o], ux = jx[o] / r, uy = jy[o] / r;
-        record[o] = __floats2half2_rn(dt, solid ? 0.0f : sqrtf(ux * ux + uy * uy));
+        const bool solid = (own_word >> (gx & 31)) & 1u;
+        const float ux = mom.y / mom.x, uy = mom.z / mom.x;
+        record[own] = __floats2half2_rn(dt, solid ? 0.0f : sqrtf(ux * ux + uy * uy));
       }
     }
     tc_before();  // the next tile's MMAs reuse the tensor memory
@@ -440,7 +502,7 @@ __global__ void __launch_bounds__(256, 2)
   __syncthreads();
   tc_after();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmemCols));
-  if (!ok && tid == 0) atomicOr(flag, 2);
+  if (!ok && lane == 0) atomicOr(flag, 2);
 }
 
 }  // namespace lbm
