@@ -67,15 +67,17 @@ constexpr long long kPadCells = 4096;
 //     15.5 against 26.7 / 12.1 against 14.4; 4096 x 2048 47 against 94 / 37
 //     against 52.  Three at once: f32 at 768 x 530 1.23 times the speed (the tile
 //     kernel 1.13), f16 at 1531 x 769 1.25.
-//   With stochastic rounding a step costs a third more: three at once were 4 %
-//     slower at 1531 x 769 and 17 % faster at 2048 x 1024; between the two
+//   With stochastic rounding a step costs a third more, and k_step_multi is
+//     the faster one only with bands of 12 rows: from 900,000 cells on (1200 x
+//     800, bf16: three at once 6.5 us a step against 7.5, alone 10.2 against
+//     13.1; 768 x 768: 5.0 against 4.5, alone 8.3 against 8.3); between the two
 //     kernels' ranges the one-step kernels stay.
 // The closure's steps run in k_step_tile: in f32 on any lattice, in 16-bit
 // storage on small ones.
 constexpr uint64_t kTileCells16 = 250000;     // k_step_tile below, 16-bit storage
 constexpr uint64_t kMultiCells32 = 400000;    // k_step_multi from here: f32 (k_step_tile below)
 constexpr uint64_t kMultiCells16 = 250000;    // 16-bit storage
-constexpr uint64_t kMultiCellsSr = 1600000;   // 16-bit storage with stochastic rounding
+constexpr uint64_t kMultiCellsSr = 900000;    // 16-bit storage with stochastic rounding
 
 size_t store_bytes(int storage) {
   switch (storage) {
@@ -600,9 +602,15 @@ template <class St> int launch_multi(lbm_sim* s) {
     // one wave of bands where that leaves 8 to 24 rows each: shorter bands
     // repeat too many halo rows (2048 x 1024, f32: 16 rows 47 us a launch, 4 rows
     // 58), taller ones wait for their last warp (4096 x 2048: 24 rows in 2.4
-    // waves 143, 59 rows in one wave 153)
-    const int bands = std::max(1, s->multi_occ * s->sms / m.wcols);
-    m.a.rows = std::min(std::max((s->L.ny + bands - 1) / bands, 8), 24);
+    // waves 143, 59 rows in one wave 153).  12 rows at least where those still
+    // fill half the slots: beside other work, 12 against 8 rows take 5.3 against
+    // 5.7 us a step (1531 x 769, f16), 6.9 against 7.8 (1024 x 1024, f32), 7.8
+    // against 9.1 (1531 x 769, bf16, stochastic rounding), alone 8.6 against 8.4,
+    // 9.8 against 9.7 and 10.5 against 10.5; with fewer cells the time alone
+    // goes up as the rows do (1024 x 512, f16: 6.8 against 5.4).
+    const int slots = s->multi_occ * s->sms, bands = std::max(1, slots / m.wcols);
+    const int least = 2 * m.wcols * ((s->L.ny + 11) / 12) >= slots ? 12 : 8;
+    m.a.rows = std::min(std::max((s->L.ny + bands - 1) / bands, least), 24);
     kern<<<m.wcols * ((s->L.ny + m.a.rows - 1) / m.a.rows), 32, smem, s->stream>>>(s->planes[s->cur], m);
   } else {
     auto kern = s->closure_on ? k_step_tile<St, false, true> : k_step_tile<St, false, false>;

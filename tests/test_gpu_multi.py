@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 # k_step_multi, just above the 400,000 cells (250,000 in 16-bit storage) from
 # which it runs: around one and two warps' 60 columns, the narrowest and the
 # lowest, bands that end unevenly
-# (stochastic rounding: four times the rows, as it starts at 1,600,000)
+# (stochastic rounding: four times the rows, as it starts at 900,000)
 SIZES = [(7, 60000), (60, 6667), (61, 6601), (62, 6452), (121, 3311), (133400, 3), (57200, 7), (1100, 370), (2521, 161)]
 # k_step_tile: tiles of 60 columns and 8 rows, or 4 where 8 leave multiprocessors idle
 SMALL = [(3, 3), (5, 4), (59, 3), (60, 8), (61, 9), (62, 12), (63, 31), (121, 40), (600, 5), (130, 700), (1200, 70),
@@ -227,4 +227,16 @@ def test_densities_of_any_scale(lbm, cuda_ok, oracle_mod, scale, ny):
     lat.iterate(5)
     o.step(5)
     np.testing.assert_array_equal(lat.populations(), o.state()[0].astype(np.float32))
+    lat.close()
+
+
+@pytest.mark.parametrize("storage,inlet,sr,nx,ny", [(0, False, None, 121, 4865), (1, False, None, 1270, 769),
+                                                    (2, True, 6, 190, 4861)])
+def test_bands_of_twelve_rows_and_a_remainder(lbm, cuda_ok, oracle_mod, storage, inlet, sr, nx, ny):
+    """Lattices whose 12-row bands fill half of the chip: the last band is short."""
+    lat, o = pair(lbm, oracle_mod, nx, ny, storage, nx, inlet, sr)
+    for n in (4, 7):
+        lat.iterate(n)
+        o.step(n)
+    same(lat, o)
     lat.close()
