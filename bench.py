@@ -7,7 +7,8 @@ inlet.  Synthetic geometry from a fixed seed; no dataset is involved.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
-A step is one fused launch over the whole grid.  `value` times K steps with the
+A launch advances the whole grid by three fused steps (the last one to three
+steps of a call, one).  `value` times K steps with the
 state resident in HBM (CUDA events on the engine's stream): the K-step call is
 first made untimed (so the CUDA graph it replays is captured and instantiated
 outside the timing), then repeated, each call bracketed by synchronisation and
@@ -48,6 +49,13 @@ def peaks():
             d = json.load(f)
         return float(d["hbm_gbs"]), "measured"
     return FALLBACK_HBM_GBS, "fallback"
+
+
+def passes_of(steps, launches):
+    """Passes over the state (every word read and written once) of a call of
+    `steps` steps: one per launch.  Fewer launches than steps mean three steps
+    a pass, with one to three single steps at the call's end."""
+    return launches if launches >= steps else (steps - 1) // 3 + (steps - 1) % 3 + 1
 
 
 def ncu_traffic(kernel_key):
@@ -296,7 +304,8 @@ def time_batched(lbm, torch, storage, steps, warmup, count=512, seed=1):
     bpc = BYTES_PER_CELL["f32" if storage == lbm.F32 else "f16"]
     return {"mlups": round(cells / (ms * 1e-3) / 1e6, 1), "mflups": round(active / (ms * 1e-3) / 1e6, 1),
             "ms_per_step": round(ms, 4), "steps": steps, "domains": count, "cells": cells,
-            "achieved_gbs": round(bpc * active / (ms * 1e-3) / 1e9, 1), "tuned": rep["chosen"],
+            "achieved_gbs": round(bpc * active / rep["chosen"]["steps_per_launch"] / (ms * 1e-3) / 1e9, 1),
+            "tuned": rep["chosen"],
             "nonfinite_domains": bad}
 
 
@@ -592,7 +601,8 @@ def run_ours(args):
         st = {"f32": lbm.F32, "f16": lbm.F16, "bf16": lbm.BF16, "f64": lbm.F64}[args.kernel_only]
         ms, launches = time_storage(lbm, torch, st, mask, args.steps, args.warmup, args.min_seconds,
                                     args.inlet_reference, args.stochastic)
-        gbs = BYTES_PER_CELL[args.kernel_only] * active / (ms * 1e-3) / 1e9
+        gbs = (BYTES_PER_CELL[args.kernel_only] * active * passes_of(args.steps, launches) /
+               (ms * args.steps * 1e-3) / 1e9)
         print(json.dumps({"kernel_only": args.kernel_only, "ms_per_step": round(ms, 5),
                           "mlups": round(n / (ms * 1e-3) / 1e6, 1), "achieved_gbs": round(gbs, 1),
                           "frac": round(gbs / hbm_peak, 4), "launches": launches}))
@@ -620,10 +630,10 @@ def run_ours(args):
     launches = (lat.launch_count() - l0 - rs.launches) // (calls + 1)
     ms_step = dev_ms / args.steps
     mlups = world * n * args.steps / (dev_ms * 1e-3) / 1e6
-    # one launch per step, replayed from a graph: the per-step device time is
-    # the launch's duration plus the graph's gap between launches
-    kernel_ms = ms_step
-    achieved = BYTES_PER_CELL["f32"] * active / (kernel_ms * 1e-3) / 1e9
+    # bytes of the launches (a launch of three steps reads and writes the state
+    # once) over the call's device time, gaps between launches included
+    passes = passes_of(args.steps, launches)
+    achieved = BYTES_PER_CELL["f32"] * active * passes / (dev_ms * 1e-3) / 1e9
     lat.close()
 
     # --- e2e: the public API with pinned host buffers, copies inside the timing --
@@ -715,8 +725,9 @@ def run_ours(args):
     variants = {}
     if not args.no_variants:
         for name, st, inlet, sr in STORAGE_RUNS[2:]:
-            vms, _ = time_storage(lbm, torch, st, mask, args.steps, args.warmup, args.min_seconds, inlet, sr)
-            gbs = BYTES_PER_CELL[name.split("_")[0]] * active / (vms * 1e-3) / 1e9
+            vms, vl = time_storage(lbm, torch, st, mask, args.steps, args.warmup, args.min_seconds, inlet, sr)
+            gbs = (BYTES_PER_CELL[name.split("_")[0]] * active * passes_of(args.steps, vl) /
+                   (vms * args.steps * 1e-3) / 1e9)
             variants[name] = {"mlups": round(n / (vms * 1e-3) / 1e6, 1), "ms_per_step": round(vms, 4),
                               "achieved_gbs": round(gbs, 1), "frac": round(gbs / hbm_peak, 4)}
 
@@ -762,11 +773,11 @@ def run_ours(args):
                 "what": "write_populations + set_mask from pinned host, K steps, read rho/ux/uy to pinned host; "
                         "median of repeated calls"},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": hbm_peak, "unit": "GB/s",
-                     "frac": round(achieved / hbm_peak, 4), "traffic": ncu_traffic("k_step_ws_f32_channel"),
+                     "frac": round(achieved / hbm_peak, 4), "traffic": ncu_traffic("k_step_multi_f32_channel"),
                      "peak_source": peak_kind, "bytes_per_cell": BYTES_PER_CELL["f32"],
                      "algorithmic_bytes_per_launch": int(BYTES_PER_CELL["f32"] * active),
-                     "active_cells": active,
-                     "kernel": "lbm::k_step_ws<StF32, EDGE_CHANNEL, NS=4, CPT=1, closure off>"},
+                     "active_cells": active, "launches_per_call": passes, "steps_per_launch": 3,
+                     "kernel": "lbm::k_step_multi<StF32, SR=0>"},
         "mflups": round(world * active * args.steps / (dev_ms * 1e-3) / 1e6, 1),
         "variants": variants,
         "batched": batched,
