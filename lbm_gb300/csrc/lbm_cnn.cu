@@ -43,7 +43,7 @@ constexpr int kTile = 64;          // pixels of a row in a convolution tile
 constexpr int kTileS = 72;         // a staged row: columns x0 - 4 .. x0 + 67 of the tile at x0, whole 16-byte words
 constexpr int kTile0 = 4;          // index of column x0 in it
 constexpr int kChunk = 8;          // input channels staged at a time
-constexpr int kWBlocks = 304;      // partial sums the weight gradient's scratch holds
+constexpr int kWBlocks = 304;      // weight-gradient blocks (2 per SM)
 constexpr int kMaxC = 32;          // channels handled by the templates
 constexpr int kLossBlocks = 608;   // loss partial sums (4 per SM)
 
@@ -129,7 +129,7 @@ __device__ __forceinline__ void mask_staged(float* sx, const float* sa, int nc, 
 // ---- 3x3 convolution to 32 channels -------------------------------------------------
 // Forward (BWD false): y = act(conv(x) + b) from C input channels.  Input
 // gradient (BWD true): the same sum over the C output channels of the layer
-// with the taps reversed, of the gradient masked by the layer's ReLU output.
+// with the pixels of the taps mirrored, of the gradient masked by the layer's ReLU output.
 // A warp owns 64 pixels of one row and all 32 channels: lane (pixel group
 // lane & 7, channel group lane >> 3) holds eight pixels (4 g .. 4 g + 3 and 32
 // further on, so that 16-byte reads do not conflict) times eight channels as
@@ -137,7 +137,8 @@ __device__ __forceinline__ void mask_staged(float* sx, const float* sa, int nc, 
 // weight pair feed: per input channel and kernel row 288 multiply-adds for
 // four reads of pixels and six of weights, where one thread per pixel read
 // eight times as many weights and was bound by those reads.  Per output the
-// terms are added in the order channel, row, column, starting from the bias.
+// terms are added in the order channel, row, column of the weights, starting
+// from the bias.
 // The next channels are copied while the current ones are summed (loading them
 // between two barriers took half the time).  4 images of 256 x 512, 32 to 32
 // channels: 195 us forward and 230 us backward; one thread per pixel took three
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(256, 2) k_conv32(const float* __restrict__ x, 
     if (BWD) {  // w [c][o][tap]
       const int c = i / (kMaxC * 9), k = i % 9;
       o = (i / 9) % kMaxC;
-      r = c * 9 + 8 - k;
+      r = c * 9 + k;
     } else {  // w [o][c][tap]
       o = i / (C * 9);
       r = i % (C * 9);
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(256, 2) k_conv32(const float* __restrict__ x, 
     for (int ci = 0; ci < nc; ci++) {
 #pragma unroll
       for (int ky = 0; ky < 3; ky++) {
-        const float* row = sx + (ci * (rows + 2) + warp + ky) * kTileS + kTile0 + 4 * pg;
+        const float* row = sx + (ci * (rows + 2) + warp + (BWD ? 2 - ky : ky)) * kTileS + kTile0 + 4 * pg;
         float v[2][6];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(256, 2) k_conv32(const float* __restrict__ x, 
                                 make_float2(wb.z, wb.w)};
 #pragma unroll
           for (int p = 0; p < 8; p++) {
-            const float2 xv = dup(v[p >> 2][(p & 3) + kx]);
+            const float2 xv = dup(v[p >> 2][(p & 3) + (BWD ? 2 - kx : kx)]);
 #pragma unroll
             for (int c = 0; c < 4; c++) acc[p][c] = __ffma2_rn(xv, wp[c], acc[p][c]);
           }
@@ -308,74 +309,81 @@ __global__ void __launch_bounds__(kTile / 4 * 8) k_conv1(const float* __restrict
 
 // ---- backward, weight gradient --------------------------------------------------
 // gw[co][ci][k] = sum over pixels of g[co] x[ci] shifted by tap k, with
-// g = ga * (a > 0) when the layer has a ReLU.  Tiles of two rows of 64 pixels
-// are staged in shared memory (g of all output channels, four input rows with
-// a 1-pixel border).  A thread holds one input channel and four output
-// channels, all nine taps, as sums over the even and the odd pixels (the
-// packed multiply-add takes two neighbouring pixels of g and of x): per four
-// pixels 72 packed multiply-adds for four reads of g, the same for the whole
-// warp, and six of x.  Half of the 16 warps take each row of a tile; CINP lanes
-// hold the input channels, and the other lanes of a warp (CINP 4) or the other
-// warps (NCOG 1: at most four output channels) take other pixels.  Their sums
-// are added in a fixed order.  One block per multiprocessor strides over tiles
-// and copies the next tile while it sums the current one; blocks leave partial
-// sums.  4 images of 256 x 512, 32 to 32 channels: 300 us.
-constexpr int kWXChan = 4 * kTileS + 4;  // 292 floats a channel: 16-byte rows, 8-byte reads of 16 lanes conflict in pairs
-constexpr int kWThreads = 512;
-template <int CINP, int NCOG> struct WGeom {
-  static constexpr int kG = 4 * NCOG * 2 * kTile, kX = CINP * kWXChan;  // floats of one tile's g, x
-  static constexpr int kTileFloats = 2 * kG + kX;                       // g, the ReLU output, x
-  static constexpr int kRed = kWThreads / 32 * 36 * 32;                 // the warps' sums at the end
-  static constexpr size_t kSmem = (size_t)(2 * kTileFloats > kRed ? 2 * kTileFloats : kRed) * sizeof(float);
+// g = ga * (a > 0) when the layer has a ReLU.  kWBlocks blocks stride over tiles
+// of 64 pixels of a row and leave partial sums; in a block every sum is one
+// chain over its pixels in order and the partials are added in block order, so
+// the result does not depend on how the threads share the sums.  A lane holds
+// one input channel (CINP 4: and one of eight groups of output channels), a
+// thread four output channels (the packed multiply-add takes two of them, which
+// lie side by side once g is masked and transposed, and one pixel of x) and KY
+// kernel rows: per four pixels of 32 to 32 channels 72 packed multiply-adds for
+// four reads of g, the same for the whole warp, and three of x.  The next tile
+// is copied while the current one is summed.  4 images of 256 x 512: 32 to 32
+// channels 287 us (a thread with 36 scalar sums, 1300), bound by the packed
+// multiply-adds' pipe; 4 to 32 97 us and 32 to 1 148 us, bound by the copies of
+// their few warps.  With the pixels of a tile shared out over more threads the
+// three took 300, 72 and 56 us, but sums in another order than before: an ulp in
+// some weights after a step.
+template <int CINP, int KY> struct WGeom {
+  static constexpr int kCO = CINP == 32 && KY == 1 ? 4 : 32;  // output channels
+  static constexpr int kThreads = KY == 3 ? 256 : 96;         // warps: groups of four output channels, or kernel rows
+  static constexpr int kGR = kTile + 4;                       // floats of a staged row of g: 17 (odd) 16-byte words
+  static constexpr int kXC = 3 * kTileS + 4;                  // floats of a channel of x: 55 16-byte words
+  static constexpr int kG = kCO * kGR, kX = CINP * kXC;       // floats of one tile's g, x
+  static constexpr int kBuf = 2 * kG + kX;                    // g, the ReLU output, x
+  static constexpr size_t kSmem = (size_t)(2 * kBuf + kTile * kCO) * sizeof(float);
 };
-template <int CINP, int NCOG>
-__global__ void __launch_bounds__(kWThreads, 1)
+template <int CINP, int KY>
+__global__ void __launch_bounds__(WGeom<CINP, KY>::kThreads, 2)
     k_conv_bwd_weight(const float* __restrict__ x, const float* __restrict__ ga, const float* __restrict__ a, int N,
                       int CIN, int COUT, int H, int W, float* __restrict__ partial) {
-  using Geo = WGeom<CINP, NCOG>;
+  using Geo = WGeom<CINP, KY>;
+  constexpr int kCO = Geo::kCO, kThreads = Geo::kThreads;
   extern __shared__ float4 smem4[];
   float* smem = (float*)smem4;
-  constexpr int kSplit = (32 / CINP) * (8 / NCOG), kSpan = kTile / kSplit;  // pixels of a row per thread
+  float* gt = smem + 2 * Geo::kBuf;  // g of the tile in work, [pixel][output channel]
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int ci = lane % CINP, rr = warp >> 3, cog = (warp & 7) % NCOG;
-  const int split = ((warp & 7) / NCOG) * (32 / CINP) + lane / CINP;
-  float2 acc[4][9];
+  const int ci = lane % CINP, cog = KY == 3 ? warp : lane / CINP, ky0 = KY == 3 ? 0 : warp;
+  // the bias sums: four channels a warp, or all of them in the first
+  const int bias_co = KY == 3 ? 4 * warp + (lane & 3) : lane % kCO;
+  const bool bias = KY == 3 || warp == 0;
+  float2 acc[2][KY][3];
 #pragma unroll
-  for (int j = 0; j < 4; j++)
+  for (int j = 0; j < 2; j++)
 #pragma unroll
-    for (int k = 0; k < 9; k++) acc[j][k] = make_float2(0.0f, 0.0f);
+    for (int k = 0; k < KY * 3; k++) acc[j][k / 3][k % 3] = make_float2(0.0f, 0.0f);
   float accb = 0.0f;
   const size_t plane = (size_t)H * W;
-  const int tiles_x = (W + kTile - 1) / kTile, tiles_y = (H + 1) / 2;
-  const long long tiles = (long long)N * tiles_y * tiles_x;
+  const int tiles_x = (W + kTile - 1) / kTile;
+  const long long tiles = (long long)N * H * tiles_x;
   const bool wide = wide_rows(ga, a, W) && wide_rows(x, nullptr, W);
   auto stage = [&](long long tile, float* G) {
     float* A = G + Geo::kG;
     float* X = A + Geo::kG;
     const int x0 = (int)(tile % tiles_x) * kTile;
     const long long rowi = tile / tiles_x;
-    const int n = (int)(rowi / tiles_y), y0 = (int)(rowi % tiles_y) * 2;
+    const int n = (int)(rowi / H), py = (int)(rowi % H);
     if (wide) {
-      for (int i = t; i < Geo::kG / 4; i += kWThreads) {
-        const int c = i / (2 * kTile / 4), yy = y0 + (i / (kTile / 4)) % 2, xx = x0 + 4 * (i % (kTile / 4));
-        const bool in = c < COUT && yy < H && xx < W;
-        const size_t o = in ? ((size_t)n * COUT + c) * plane + (size_t)yy * W + xx : 0;
-        copy16(G + 4 * i, ga + o, in);
-        if (a) copy16(A + 4 * i, a + o, in);
+      for (int i = t; i < kCO * (kTile / 4); i += kThreads) {
+        const int c = i / (kTile / 4), p = 4 * (i % (kTile / 4));
+        const bool in = c < COUT && x0 + p < W;
+        const size_t o = in ? ((size_t)n * COUT + c) * plane + (size_t)py * W + x0 + p : 0;
+        copy16(G + c * Geo::kGR + p, ga + o, in);
+        if (a) copy16(A + c * Geo::kGR + p, a + o, in);
       }
     } else {
-      for (int i = t; i < Geo::kG; i += kWThreads) {
-        const int c = i / (2 * kTile), yy = y0 + (i / kTile) % 2, xx = x0 + i % kTile;
-        const bool in = c < COUT && yy < H && xx < W;
-        const size_t o = in ? ((size_t)n * COUT + c) * plane + (size_t)yy * W + xx : 0;
-        copy4(G + i, ga + o, in);
-        if (a) copy4(A + i, a + o, in);
+      for (int i = t; i < kCO * kTile; i += kThreads) {
+        const int c = i / kTile, p = i % kTile;
+        const bool in = c < COUT && x0 + p < W;
+        const size_t o = in ? ((size_t)n * COUT + c) * plane + (size_t)py * W + x0 + p : 0;
+        copy4(G + c * Geo::kGR + p, ga + o, in);
+        if (a) copy4(A + c * Geo::kGR + p, a + o, in);
       }
     }
-    for (int r = warp; r < CINP * 4; r += kWThreads / 32) {
-      const int c = r >> 2, yy = y0 + (r & 3) - 1;
+    for (int r = warp; r < CINP * 3; r += kThreads / 32) {
+      const int c = r / 3, yy = py + r % 3 - 1;
       const bool row_in = c < CIN && yy >= 0 && yy < H;
-      stage_row(X + c * kWXChan + (r & 3) * kTileS, x + (row_in ? ((size_t)n * CIN + c) * plane + (size_t)yy * W : 0),
+      stage_row(X + c * Geo::kXC + (r % 3) * kTileS, x + (row_in ? ((size_t)n * CIN + c) * plane + (size_t)yy * W : 0),
                 row_in, x0, W, wide);
     }
     copies_commit();
@@ -383,113 +391,100 @@ __global__ void __launch_bounds__(kWThreads, 1)
   int turn = 0;
   if (blockIdx.x < tiles) stage(blockIdx.x, smem);
   for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x, turn ^= 1) {
-    float* G = smem + turn * Geo::kTileFloats;
+    const float* G = smem + turn * Geo::kBuf;
     const float* X = G + 2 * Geo::kG;
     if (tile + gridDim.x < tiles) {
-      stage(tile + gridDim.x, smem + (turn ^ 1) * Geo::kTileFloats);
+      stage(tile + gridDim.x, smem + (turn ^ 1) * Geo::kBuf);
       copies_wait<1>();
     } else {
       copies_wait<0>();
     }
-    if (a) {  // (each thread masks its own copies)
-      if (wide) {
-        for (int i = t; i < Geo::kG / 4; i += kWThreads) {
-          float4 g = ((float4*)G)[i];
-          const float4 q = ((const float4*)(G + Geo::kG))[i];
-          if (!(q.x > 0.0f)) g.x = 0.0f;
-          if (!(q.y > 0.0f)) g.y = 0.0f;
-          if (!(q.z > 0.0f)) g.z = 0.0f;
-          if (!(q.w > 0.0f)) g.w = 0.0f;
-          ((float4*)G)[i] = g;
-        }
-      } else {
-        for (int i = t; i < Geo::kG; i += kWThreads)
-          if (!(G[Geo::kG + i] > 0.0f)) G[i] = 0.0f;
+    __syncthreads();
+    for (int i = t; i < kCO * (kTile / 4); i += kThreads) {
+      const int co = i % kCO, p = 4 * (i / kCO);
+      float4 g = *(const float4*)(G + co * Geo::kGR + p);
+      if (a) {
+        const float4 q = *(const float4*)(G + Geo::kG + co * Geo::kGR + p);
+        if (!(q.x > 0.0f)) g.x = 0.0f;
+        if (!(q.y > 0.0f)) g.y = 0.0f;
+        if (!(q.z > 0.0f)) g.z = 0.0f;
+        if (!(q.w > 0.0f)) g.w = 0.0f;
       }
+      gt[p * kCO + co] = g.x;
+      gt[(p + 1) * kCO + co] = g.y;
+      gt[(p + 2) * kCO + co] = g.z;
+      gt[(p + 3) * kCO + co] = g.w;
     }
     __syncthreads();
-    if (t < 4 * NCOG * 16) {  // bias: 16 threads per output channel
+    const float* gp = gt + 4 * cog;
+    const float* xp = X + ci * Geo::kXC + ky0 * kTileS + kTile0;
+    float before[KY];  // pixel p - 1 of each row
+    float4 now[KY];    // pixels p .. p + 3
 #pragma unroll
-      for (int i = 0; i < 2 * kTile / 16; i++) accb += G[(t >> 4) * 2 * kTile + (t & 15) + 16 * i];
+    for (int ky = 0; ky < KY; ky++) {
+      before[ky] = xp[ky * kTileS - 1];
+      now[ky] = *(const float4*)(xp + ky * kTileS);
     }
-    const float* gp = G + (4 * cog * 2 + rr) * kTile + split * kSpan;
-    const float* xp = X + ci * kWXChan + rr * kTileS + kTile0 + split * kSpan;
-    // pixels p, p + 1 of the three rows, and p - 1, p
-    float2 x2[3], left[3];
+#pragma unroll 1
+    for (int p = 0; p < kTile; p += 4) {
+      float4 g[4];
 #pragma unroll
-    for (int ky = 0; ky < 3; ky++) {
-      x2[ky] = *(const float2*)(xp + ky * kTileS);
-      left[ky] = make_float2(xp[ky * kTileS - 1], x2[ky].x);
-    }
-#pragma unroll 2
-    for (int p = 0; p < kSpan; p += 4) {
-      float4 g4[4];
+      for (int i = 0; i < 4; i++) g[i] = *(const float4*)(gp + (p + i) * kCO);
+      if (bias) {
 #pragma unroll
-      for (int j = 0; j < 4; j++) g4[j] = *(const float4*)(gp + j * 2 * kTile + p);
+        for (int i = 0; i < 4; i++) accb += gt[(p + i) * kCO + bias_co];
+      }
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
+      for (int ky = 0; ky < KY; ky++) {
+        const float4 next = *(const float4*)(xp + ky * kTileS + p + 4);
+        const float v[6] = {before[ky], now[ky].x, now[ky].y, now[ky].z, now[ky].w, next.x};
 #pragma unroll
-        for (int ky = 0; ky < 3; ky++) {
-          const float2 nx = *(const float2*)(xp + ky * kTileS + p + 2 * h + 2);
-          const float2 right = make_float2(x2[ky].y, nx.x);
+        for (int i = 0; i < 4; i++)
 #pragma unroll
           for (int kx = 0; kx < 3; kx++) {
-            const float2 xv = kx == 0 ? left[ky] : (kx == 1 ? x2[ky] : right);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-              const float2 g = h ? make_float2(g4[j].z, g4[j].w) : make_float2(g4[j].x, g4[j].y);
-              acc[j][ky * 3 + kx] = __ffma2_rn(xv, g, acc[j][ky * 3 + kx]);
-            }
+            const float2 xv = dup(v[i + kx]);
+            acc[0][ky][kx] = __ffma2_rn(xv, make_float2(g[i].x, g[i].y), acc[0][ky][kx]);
+            acc[1][ky][kx] = __ffma2_rn(xv, make_float2(g[i].z, g[i].w), acc[1][ky][kx]);
           }
-          left[ky] = right;
-          x2[ky] = nx;
-        }
+        before[ky] = now[ky].w;
+        now[ky] = next;
       }
     }
     __syncthreads();  // this buffer takes the tile after the next
   }
   const int nw = COUT * CIN * 9;
   float* part = partial + (size_t)blockIdx.x * (nw + COUT);
-  if (t < 4 * NCOG * 16) {  // (whole warps)
-    for (int d = 1; d < 16; d <<= 1) accb += __shfl_xor_sync(0xffffffffu, accb, d);
-    if ((t & 15) == 0 && (t >> 4) < COUT) part[nw + (t >> 4)] = accb;
-  }
+  if (ci < CIN) {
 #pragma unroll
-  for (int j = 0; j < 4; j++)
+    for (int j = 0; j < 4; j++) {
+      const int co = 4 * cog + j;
+      if (co >= COUT) break;
 #pragma unroll
-    for (int k = 0; k < 9; k++) {
-      float s = acc[j][k].x + acc[j][k].y;
+      for (int ky = 0; ky < KY; ky++)
 #pragma unroll
-      for (int d = CINP; d < 32; d <<= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-      smem[(warp * 36 + j * 9 + k) * 32 + lane] = s;
+        for (int kx = 0; kx < 3; kx++)
+          part[(co * CIN + ci) * 9 + (ky0 + ky) * 3 + kx] = (j & 1) ? acc[j >> 1][ky][kx].y : acc[j >> 1][ky][kx].x;
     }
-  __syncthreads();
-  // sum over the warps that share a group of output channels
-  for (int i = t; i < NCOG * 36 * CINP; i += kWThreads) {
-    const int c = i % CINP, e = (i / CINP) % 36, g = i / (CINP * 36), co = 4 * g + e / 9;
-    float s = 0.0f;
-#pragma unroll
-    for (int v = 0; v < kWThreads / 32; v += NCOG) s += smem[((v + g) * 36 + e) * 32 + c];
-    if (co < COUT && c < CIN) part[(co * CIN + c) * 9 + e % 9] = s;
   }
+  if (bias && lane < (KY == 3 ? 4 : kCO) && bias_co < COUT) part[nw + bias_co] = accb;
 }
 
-// Sum the per-block partials [nblocks][nw + nb] into the weight gradient
-// (first nw entries) and the bias gradient (last nb): eight threads per entry
-// add a run of blocks each, and their sums are added in order.
+// Sum the per-block partials [nblocks][nw + nb] in block order into the weight
+// gradient (first nw entries) and the bias gradient (last nb): eight warps
+// fetch 32 entries of all blocks, and one lane per entry adds them.
 __global__ void __launch_bounds__(256) k_sum_partials(const float* __restrict__ partial, int nblocks, int nw, int nb,
                                                       float* __restrict__ gw, float* __restrict__ gb) {
-  __shared__ float sh[8][32];
-  const int i = blockIdx.x * 32 + (threadIdx.x & 31), seg = threadIdx.x >> 5, n = nw + nb;
-  const int per = (nblocks + 7) / 8, b1 = min(nblocks, (seg + 1) * per);
-  float s = 0.0f;
-  if (i < n)
-    for (int bl = seg * per; bl < b1; bl++) s += partial[(size_t)bl * n + i];
-  sh[seg][threadIdx.x & 31] = s;
+  __shared__ float sh[kWBlocks][32];
+  const int lane = threadIdx.x & 31, i = blockIdx.x * 32 + lane, n = nw + nb;
+  if (i < n) {
+#pragma unroll 8
+    for (int bl = threadIdx.x >> 5; bl < nblocks; bl += 8) sh[bl][lane] = partial[(size_t)bl * n + i];
+  }
   __syncthreads();
-  if (seg != 0 || i >= n) return;
-#pragma unroll
-  for (int k = 1; k < 8; k++) s += sh[k][threadIdx.x];
+  if (threadIdx.x >= 32 || i >= n) return;
+  float s = 0.0f;
+#pragma unroll 8
+  for (int bl = 0; bl < nblocks; bl++) s += sh[bl][lane];
   if (i < nw) gw[i] = s;
   else gb[i - nw] = s;
 }
@@ -692,13 +687,14 @@ int launch_conv32(bool bwd, const float* x, const float* a, int n, int C, int h,
   return LBM_OK;
 }
 
-template <int CINP, int NCOG>
+template <int CINP, int KY>
 int launch_bwd_weight(const float* in, const float* grad_out, const float* out, int n, int cin, int cout, int h, int w,
                       float* scratch, int blocks, cudaStream_t s) {
-  constexpr size_t smem = WGeom<CINP, NCOG>::kSmem;
-  auto kern = k_conv_bwd_weight<CINP, NCOG>;
+  using Geo = WGeom<CINP, KY>;
+  constexpr size_t smem = Geo::kSmem;
+  auto kern = k_conv_bwd_weight<CINP, KY>;
   CCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<blocks, kWThreads, smem, s>>>(in, grad_out, out, n, cin, cout, h, w, scratch);
+  kern<<<blocks, Geo::kThreads, smem, s>>>(in, grad_out, out, n, cin, cout, h, w, scratch);
   CCK(cudaGetLastError());
   return LBM_OK;
 }
@@ -739,11 +735,11 @@ int lbm_cnn_conv_backward_weight(const float* in, const float* grad_out, const f
   if (scratch_bytes < (size_t)kWBlocks * per * sizeof(float))
     return cfail(LBM_ERR_ARG, "scratch needs %zu bytes", (size_t)kWBlocks * per * sizeof(float));
   cudaStream_t s = as_stream(stream);
-  const long long tiles = (long long)n * ((h + 1) / 2) * ((w + kTile - 1) / kTile);
-  const int blocks = (int)(tiles < kWBlocks / 2 ? tiles : kWBlocks / 2);  // one per multiprocessor at most
-  const int rc = cout <= 4 ? launch_bwd_weight<32, 1>(in, grad_out, out, n, cin, cout, h, w, scratch, blocks, s)
-                 : cin <= 4 ? launch_bwd_weight<4, 8>(in, grad_out, out, n, cin, cout, h, w, scratch, blocks, s)
-                            : launch_bwd_weight<32, 8>(in, grad_out, out, n, cin, cout, h, w, scratch, blocks, s);
+  const long long tiles = (long long)n * h * ((w + kTile - 1) / kTile);
+  const int blocks = (int)(tiles < kWBlocks ? tiles : kWBlocks);
+  const int rc = cin <= 4    ? launch_bwd_weight<4, 1>(in, grad_out, out, n, cin, cout, h, w, scratch, blocks, s)
+                 : cout <= 4 ? launch_bwd_weight<32, 1>(in, grad_out, out, n, cin, cout, h, w, scratch, blocks, s)
+                             : launch_bwd_weight<32, 3>(in, grad_out, out, n, cin, cout, h, w, scratch, blocks, s);
   if (rc) return rc;
   k_sum_partials<<<(per + 31) / 32, 256, 0, s>>>(scratch, blocks, nw, cout, grad_weight, grad_bias);
   CCK(cudaGetLastError());
