@@ -104,11 +104,12 @@ int lbm_get_stream(const lbm_sim* sim, void** cuda_stream);
  * strip (channel mode with f16 / bf16 storage; otherwise as 8); 11, 12, 13:
  * rings of 5, 6, 7 stages, two cells per thread and 512-column strips
  * (channel mode with f16 / bf16 storage; otherwise as 7).  Defaults: 3
- * for f32, 11 for f16 / bf16 (7 below 1024 columns), with rows_per_thread 8 for kernels 0 / 1 and a
- * band floor of 2 rows for the staged kernels; f64 storage always uses
- * kernel 0.  Until this is called, lbm_step takes three steps per launch
- * where it can (channel mode below f64); the chosen kernel then takes every
- * step by itself.  No counterpart in the reference, whose dispatch is fixed at
+ * for f32, 11 for f16 / bf16 (7 below 1024 columns), with rows_per_thread 8
+ * for kernel 1, 1 for kernel 0 and a band floor of 2 rows for the staged
+ * kernels; f64 storage always uses kernel 0.  Until this is called, lbm_step
+ * takes three steps per launch where it can (channel mode below f64) and two
+ * cells per thread in reference mode; the chosen kernel then takes every step
+ * by itself.  No counterpart in the reference, whose dispatch is fixed at
  * 256-wide 1-D workgroups (lbm.rs:102-106). */
 int lbm_set_tuning(lbm_sim* sim, int rows_per_thread, int kernel);
 

@@ -9,7 +9,9 @@
 // dealt round-robin) or dynamically (an atomic ticket per tile).  Which ring
 // depth, cells per thread, schedule and band height per domain-height bucket
 // to use is chosen by lbm_batch_autotune, which times the candidates on the
-// batch itself.
+// batch itself.  Batches of kMultiCells or more take three steps per launch
+// (k_batch_multi, one warp per tile of 60 columns) and use the staged step for
+// a call's last ones.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdarg>
@@ -273,6 +275,8 @@ struct lbm_batch {
   CUtensorMap* d_maps = nullptr;  // two per domain: the 8 planes of each buffer set
   int4* d_mtiles = nullptr;       // tiles of the three-step launches
   int nmtiles = 0, rest_i = 0;    // their number; the rest planes that hold the state
+  bool captured = false;          // the caller captured steps: one step per launch from then on, as the
+                                  // captured launches hold the addresses of the rest planes
   int* d_counter = nullptr;  // one ticket counter per step of a captured graph
   int counters_cap = 0;
   int* d_flag = nullptr;
@@ -377,7 +381,9 @@ size_t multi_smem(int storage) {
   return storage == STORE_F32 ? (size_t)MultiGeom<float>::kStages * MultiGeom<float>::kBytes
                               : (size_t)MultiGeom<__half>::kStages * MultiGeom<__half>::kBytes;
 }
-bool multi_default(const lbm_batch* b) { return b->cells >= (b->sr_on ? kMultiCellsSr : kMultiCells); }
+bool multi_default(const lbm_batch* b) {
+  return !b->captured && b->cells >= (b->sr_on ? kMultiCellsSr : kMultiCells);
+}
 
 // Tensor maps and tiles of the three-step launches: bands of 8 to 24 rows, as
 // many as one wave of CTAs takes (the single lattice's rule over all domains).
@@ -776,6 +782,13 @@ int lbm_batch_init_equilibrium(lbm_batch* b, float noise_amp, uint64_t seed) {
 int lbm_batch_step(lbm_batch* b, uint32_t n) {
   if (!b) return bfail(LBM_ERR_ARG, "null batch");
   int rc;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  BCK(cudaStreamIsCapturing(b->stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) {
+    b->captured = true;
+    if (b->cfg.multi) drop_graphs(b);
+    b->cfg.multi = false;
+  }
   for (uint32_t k = 0; k < n;) {
     const uint32_t left = n - k;
     const bool last = left == 1;
@@ -1017,8 +1030,8 @@ int lbm_batch_autotune(lbm_batch* b, uint32_t steps_per_trial, char* report, siz
   }
   // stage 3: three steps per launch, the schedule above for the other steps
   b->cfg = best_cfg;
-  b->cfg.multi = true;
-  int rc = trial("three_steps", &best, &best_cfg);
+  b->cfg.multi = !b->captured;
+  int rc = b->captured ? LBM_OK : trial("three_steps", &best, &best_cfg);
   if (rc) return rc;
   b->cfg = best_cfg;
   rc = configure(b);

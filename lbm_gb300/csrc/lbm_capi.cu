@@ -153,6 +153,10 @@ struct lbm_sim {
   int rest_parity = 0;      // flips each time the two rest planes change places
   bool inlet_same = true;   // both buffer sets hold the same words in column 0
   bool tuned = false;       // lbm_set_tuning chose the step kernel
+  // The caller captured work on this handle: its graph holds the addresses of
+  // the rest plane that was current then, so from then on every step is one
+  // launch (the rest planes change places no more).
+  bool captured = false;
   CUtensorMap planes[2] = {};  // the 8 planes of each buffer set, for its copies
   int multi_occ = 0, multi_variant = -1;  // three-step kernel: CTAs per multiprocessor, for which variant
   void* mask_base = nullptr;
@@ -169,10 +173,6 @@ struct lbm_sim {
   cudaStream_t own_stream = nullptr, stream = nullptr;
   int cur = 0;               // buffer holding the latest state
   bool materialised = true;  // cur holds a pre-collision state
-  // the populations were read from the fused representation since the last
-  // step: a checkpoint, or a call on rows, made now sees the pre-collision
-  // state, as if the read had left it (a step leaves the same words either way)
-  bool pulled_read = false;
   bool moments_valid = false;
   uint64_t steps = 0, launches = 0;
   int rows = 0;    // rows per thread / band floor; 0: 8 for the per-cell kernels, 2 for the staged ones
@@ -305,9 +305,19 @@ void default_walls(lbm_sim* s) {
   }
 }
 
+// Whether the caller is capturing the handle's stream; remembered in `captured`.
+int note_capture(lbm_sim* s, bool* now = nullptr) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (s->stream != nullptr) CK(cudaStreamIsCapturing(s->stream, &st));
+  if (st != cudaStreamCaptureStatusNone) s->captured = true;
+  if (now) *now = st != cudaStreamCaptureStatusNone;
+  return LBM_OK;
+}
+
 // Bring the reference's pre-collision state S_k into buffer `cur`.
 int materialise(lbm_sim* s) {
   if (s->materialised) return LBM_OK;
+  if (int rc = note_capture(s)) return rc;
   const int dst = 1 - s->cur;
   dim3 grid((s->L.nx + kBlockX - 1) / kBlockX, s->L.ny);
   const StoreRef ref = store_ref(s);
@@ -328,7 +338,6 @@ int materialise(lbm_sim* s) {
   s->launches++;
   s->cur = dst;
   s->materialised = true;
-  s->pulled_read = false;
   return LBM_OK;
 }
 
@@ -361,7 +370,6 @@ int launch_init(lbm_sim* s, double rho, double ux, double uy, double amp, uint64
   s->launches++;
   s->cur = 0;
   s->materialised = true;
-  s->pulled_read = false;
   s->moments_valid = false;
   s->inlet_same = true;
   s->steps = 0;
@@ -567,10 +575,11 @@ int three_kernel(const lbm_sim* s) {
 }
 // Whether a call may take three steps in one launch: the lattice's default
 // kernel, a state past its first step (a materialised one is collided in
-// place), and the same words in column 0 of both buffer sets (the levels of a
-// launch pull the inlet from one of them).
+// place), the same words in column 0 of both buffer sets (the levels of a
+// launch pull the inlet from one of them), and no graph of the caller's that
+// holds one of the rest planes.
 bool multi_ok(const lbm_sim* s) {
-  return s->rest_out && !s->tuned && !s->materialised && s->inlet_same && three_kernel(s) != THREE_NONE;
+  return s->rest_out && !s->tuned && !s->captured && !s->materialised && s->inlet_same && three_kernel(s) != THREE_NONE;
 }
 int multi_key(const lbm_sim* s) { return 4 * three_kernel(s) + (s->closure_on ? 2 : 0) + (s->sr_on ? 1 : 0); }
 
@@ -630,6 +639,7 @@ template <class St> int launch_multi(lbm_sim* s) {
 }
 
 int compute_moments(lbm_sim* s) {
+  if (int rc = note_capture(s)) return rc;
   dim3 grid((s->L.nx + kBlockX - 1) / kBlockX, s->L.ny);
   auto launch = [&](auto tag) -> int {
     using St = decltype(tag);
@@ -1074,7 +1084,6 @@ static int launch_step(lbm_sim* s, bool last) {
   if (rc) return rc;
   s->cur = dst;
   s->materialised = false;
-  s->pulled_read = false;
   s->steps++;
   if (s->sr_on) s->clock_pending++;
   return LBM_OK;
@@ -1097,7 +1106,6 @@ static int launch_steps3(lbm_sim* s) {
   s->launches++;
   s->cur = 1 - s->cur;
   swap_rest(s);
-  s->pulled_read = false;
   s->steps += kMultiSteps;
   if (s->sr_on) s->clock_pending += kMultiSteps;
   return LBM_OK;
@@ -1198,7 +1206,6 @@ static int replay_steps(lbm_sim* s, StepRun* runs, uint32_t n, bool moments) {
   }
   if ((rc = advance_clock(s))) return rc;
   CK(cudaGraphLaunch(run.exec, s->stream));
-  s->pulled_read = false;
   s->steps += n;
   s->launches += run.launches;
   s->cur ^= (int)(n & 1u);
@@ -1213,10 +1220,10 @@ int lbm_step(lbm_sim* s, uint32_t n) {
   // once the launch shapes are known (the legacy default stream cannot be
   // captured): a short call repeated with the same length replays one graph
   // of the whole call; longer calls replay runs of kStepGraph steps.
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;  // a caller's own capture: plain launches
-  if (s->stream != nullptr) CK(cudaStreamIsCapturing(s->stream, &capturing));
+  bool capturing = false;  // a caller's own capture: plain launches
+  if (int rc = note_capture(s, &capturing)) return rc;
   auto steady = [&]() {
-    return s->use_graphs && s->stream != nullptr && capturing == cudaStreamCaptureStatusNone && !s->materialised &&
+    return s->use_graphs && s->stream != nullptr && !capturing && !s->materialised &&
            (s->storage == STORE_F64 || s->kernel < 2 || pair_ok(s) ||
             s->staged_variant == staged_key(s->kernel, s->closure_on, s->sr_on != 0u)) &&
            (n <= (uint32_t)kMultiSteps || !multi_ok(s) || s->multi_variant == multi_key(s));
@@ -1246,11 +1253,8 @@ int lbm_step_rows(lbm_sim* s, uint32_t y0, uint32_t y1, int flags) {
   CHECK_SIM_ANY(s);
   if (y0 >= y1 || y1 > (uint32_t)s->L.ny || (flags & ~(LBM_ROWS_COMPLETE | LBM_ROWS_MOMENTS)))
     return fail(LBM_ERR_ARG, "rows %u..%u of %d, flags 0x%x", y0, y1, s->L.ny, flags);
+  if (int rc = note_capture(s)) return rc;
   if (s->pending < 0) {
-    if (s->pulled_read) {
-      int rc = materialise(s);
-      if (rc) return rc;
-    }
     s->pending = s->materialised ? s->cur : 1 - s->cur;
     s->pending_moments = true;
   }
@@ -1262,7 +1266,6 @@ int lbm_step_rows(lbm_sim* s, uint32_t y0, uint32_t y1, int flags) {
     s->cur = s->pending;
     s->pending = -1;
     s->materialised = false;
-    s->pulled_read = false;
     s->steps++;
     s->moments_valid = s->pending_moments;
     if (s->sr_on) s->clock_pending++;  // every row range of the step read the same index
@@ -1334,6 +1337,8 @@ int lbm_read_field_device(lbm_sim* s, int field, float* device_out) { return rea
 static int read_pops(lbm_sim* s, void* out, bool f64, bool device_out = false) {
   CHECK_SIM(s);
   if (!out) return fail(LBM_ERR_ARG, "out is null");
+  int rc = note_capture(s);
+  if (rc) return rc;
   dim3 grid((s->L.nx + kBlockX - 1) / kBlockX, s->L.ny);
   void* mapped = device_out ? nullptr : mapped_host(out);
   void* dst = device_out ? out : (mapped ? mapped : (void*)s->staging_d);
@@ -1342,24 +1347,26 @@ static int read_pops(lbm_sim* s, void* out, bool f64, bool device_out = false) {
     using S = typename St::S;
     using O = std::remove_pointer_t<decltype(o)>;
     const StoreRef ref = store_ref(s);
-    const S *cur = (const S*)s->f[s->cur], *old = (const S*)s->f[1 - s->cur], *rest = (const S*)s->rest;
+    const S *cur = (const S*)s->f[s->cur], *rest = (const S*)s->rest;
+    S* other = (S*)s->f[1 - s->cur];
     if (s->materialised)
       k_read_pops<St, O><<<grid, kBlockX, 0, s->stream>>>(s->L, cur, rest, o, ref);
     else if (s->edge == EDGE_REF)
-      k_read_pops_pulled<St, EDGE_REF, O><<<grid, kBlockX, 0, s->stream>>>(s->L, cur, old, rest, s->mask_d, o, ref);
+      k_materialise_read<St, EDGE_REF, O><<<grid, kBlockX, 0, s->stream>>>(s->L, cur, other, rest, s->mask_d, o, ref);
     else
-      k_read_pops_pulled<St, EDGE_CHANNEL, O><<<grid, kBlockX, 0, s->stream>>>(s->L, cur, old, rest, s->mask_d, o, ref);
+      k_materialise_read<St, EDGE_CHANNEL, O><<<grid, kBlockX, 0, s->stream>>>(s->L, cur, other, rest, s->mask_d, o,
+                                                                                ref);
     CK_LAUNCH();
     return LBM_OK;
   };
   auto launch = [&](auto tag) -> int {
     return f64 ? launch_as(tag, (double*)dst) : launch_as(tag, (float*)dst);
   };
-  s->pulled_read = !s->materialised;
-  int rc;
   rc = dispatch_storage(s->storage, launch);
   if (rc) return rc;
   s->launches++;
+  if (!s->materialised) s->cur = 1 - s->cur;
+  s->materialised = true;
   if (device_out) return LBM_OK;
   if (!mapped)
     CK(cudaMemcpyAsync(out, s->staging_d, (size_t)9 * s->L.nx * s->L.ny * (f64 ? 8 : 4), cudaMemcpyDeviceToHost,
@@ -1410,7 +1417,6 @@ static int write_pops(lbm_sim* s, const void* in, bool f64) {
   if (rc) return rc;
   s->cur = 0;
   s->materialised = true;
-  s->pulled_read = false;
   s->moments_valid = false;
   s->inlet_same = true;
   s->steps = 0;
@@ -1765,7 +1771,6 @@ int lbm_checkpoint_save(lbm_sim* s, void* buf, size_t len) {
   const size_t need = sizeof(CkHeader) + ck_payload_bytes(s, closure);
   if (!buf || len < need) return fail(LBM_ERR_ARG, "checkpoint needs %zu bytes", need);
   int rc = ensure_mask_host(s);
-  if (!rc && s->pulled_read) rc = materialise(s);
   if (rc) return rc;
   const size_t cells = (size_t)s->L.nx * s->L.ny, e = s->es;
   CkHeader h{};
@@ -1897,7 +1902,6 @@ int lbm_checkpoint_load(lbm_sim* s, const void* buf, size_t len) {
   s->steps = h.steps;
   s->cur = (int)h.cur;
   s->materialised = h.materialised != 0;
-  s->pulled_read = false;
   s->moments_valid = false;
   s->inlet_same = true;  // column 0 of the two buffer sets
   for (size_t row = 0; row < 8 * (size_t)s->L.ny && s->inlet_same; row++)
@@ -1944,10 +1948,6 @@ static int rows_io(lbm_sim* s, uint32_t y, uint32_t nrows, uint32_t slot_mask, v
   // y >= ny || nrows > ny - y: no sum that could wrap in 32 bits
   if (nrows == 0 || y >= (uint32_t)s->L.ny || nrows > (uint32_t)s->L.ny - y || slot_mask == 0 || slot_mask > 0xFFu)
     return fail(LBM_ERR_ARG, "rows %u (+%u) of %d, slot mask 0x%x", y, nrows, s->L.ny, slot_mask);
-  if (s->pulled_read) {
-    int rc = materialise(s);
-    if (rc) return rc;
-  }
   const size_t e = s->es, row = (size_t)s->L.nx * e;
   const cudaMemcpyKind kind = read ? (on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost)
                                    : (on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);

@@ -545,8 +545,7 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
 // coarse solid flag (fewer than half the cells fluid).  FIXED: the factor, its
 // block's moments kept in registers between the two sweeps (every population is
 // then read once, F at a time); 0: any factor, read twice.  Bound by memory (36
-// bytes a fine cell).  With populations read without materialising them, three
-// samples of a 2048 x 1024 run (forty steps) went from 357 to 314 us.
+// bytes a fine cell).
 template <int FIXED>
 __global__ void k_coarsen(const float* __restrict__ pops, const uint8_t* __restrict__ solid_f, int Hf, int Wf,
                           int factor, float* __restrict__ avg, uint8_t* __restrict__ solid_c) {

@@ -498,17 +498,15 @@ __global__ void k_read_pops(Layout L, const typename St::S* f, const typename St
   }
 }
 
-// The same populations read from the fused representation (src: P_k, old: the
-// other buffer set): pulled with bounce-back, a bounced 16-bit word rounded for
-// its new direction, or the cell's own previous words where it is not streamed,
-// which is what k_materialise would leave behind, without writing it.  Bound by
-// memory: a read is one pass of 72 bytes a cell where materialising first was
-// two of 136, and the steps after it go on from the fused state (the first
-// step from a materialised one is a launch of its own, in place).
+// The same populations read from the fused representation, materialised in the
+// same pass (k_materialise: src is P_k, dst the other buffer set, whose cells
+// that are not streamed keep their words): pulled with bounce-back, a bounced
+// 16-bit word rounded for its new direction.  Bound by memory: reading what had
+// been materialised first took 4 bytes in 17 more (f32).
 template <class St, int EDGE, class O>
-__global__ void k_read_pops_pulled(Layout L, const typename St::S* __restrict__ src,
-                                   const typename St::S* __restrict__ old, const typename St::S* __restrict__ rest,
-                                   const uint32_t* __restrict__ mask, O* __restrict__ out, StoreRef ref) {
+__global__ void k_materialise_read(Layout L, const typename St::S* __restrict__ src, typename St::S* dst,
+                                   const typename St::S* __restrict__ rest, const uint32_t* __restrict__ mask,
+                                   O* __restrict__ out, StoreRef ref) {
   using S = typename St::S;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y;
@@ -517,20 +515,25 @@ __global__ void k_read_pops_pulled(Layout L, const typename St::S* __restrict__ 
   const long long n = (long long)L.nx * L.ny, c = (long long)y * L.nx + x;
   const bool still = mask_bit(mask, L.mw, x, y) || x == 0 || (EDGE == EDGE_REF && y == L.ny - 1);
   const bool interior = x >= 1 && x <= L.nx - 2 && y >= 1 && y <= L.ny - 2;
+  S v[9];
 #pragma unroll
   for (int q = 0; q < 9; q++) {
-    S v;
     if (q == 4) {
-      v = rest[own];
+      v[q] = rest[own];
     } else if (still) {
-      v = old[(long long)slot(q) * L.ps + own];
+      v[q] = dst[(long long)slot(q) * L.ps + own];
     } else {
       int ux_ = x - cx(q), uy_ = y - cy(q);
       if (!interior) upstream_edge<EDGE>(L, x, y, q, ux_, uy_);
-      v = mask_bit(mask, L.mw, ux_, uy_) ? St::store(St::bounce(src[(long long)slot(8 - q) * L.ps + own], q, ref), q)
-                                         : src[(long long)slot(q) * L.ps + (long long)uy_ * L.pitch + ux_];
+      v[q] = mask_bit(mask, L.mw, ux_, uy_)
+                 ? St::store(St::bounce(src[(long long)slot(8 - q) * L.ps + own], q, ref), q)
+                 : src[(long long)slot(q) * L.ps + (long long)uy_ * L.pitch + ux_];
     }
-    out[q * n + c] = (O)St::f_of(v, q, ref);
+  }
+#pragma unroll
+  for (int q = 0; q < 9; q++) {
+    out[q * n + c] = (O)St::f_of(v[q], q, ref);
+    if (q != 4 && !still) dst[(long long)slot(q) * L.ps + own] = v[q];
   }
 }
 

@@ -1,4 +1,7 @@
-// Staged, warp-specialised fused step (the default step kernel).
+// Staged, warp-specialised fused step: one step per launch in channel mode, where
+// three steps per launch do not apply (a call's last steps, a state's first, row
+// ranges, 16-bit storage with stochastic rounding or the closure at middle
+// sizes), and wherever lbm_set_tuning chose it.
 //
 // A CTA owns a strip of W columns (kStageW = 256, or 512 for 16-bit storage)
 // and a contiguous band of rows.  One producer warp moves row segments of

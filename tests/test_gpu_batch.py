@@ -298,3 +298,38 @@ def test_gpu_batch_three_step_launches_match_oracle_per_domain(lbm, cuda_ok, ora
             assert_domain(b, d, orc[d])
         b.synchronize()
         assert b.info()[2] == done
+
+
+def test_a_callers_graph_of_batch_steps_survives_other_steps(lbm, cuda_ok):
+    """Ten steps captured by the caller on the batch's stream and replayed
+    around plain calls, against as many plain steps."""
+    import torch
+    from lbm_gb300 import batch as B
+    nx, ny = np.array([700, 640]), np.array([320, 350])
+    om, u = np.array([1.5, 1.7], np.float32), np.array([0.05, 0.04], np.float32)
+    rng = np.random.default_rng(3)
+    masks = [(rng.random((y, x)) < 0.05).astype(np.uint8) for x, y in zip(nx, ny)]
+
+    def batch():
+        b = B.Batch(nx, ny, om, u, lbm.F32)
+        for d, m in enumerate(masks):
+            b.set_mask(d, m)
+        b.init_equilibrium(1e-3, 4)
+        return b
+
+    a, c = batch(), batch()
+    a.step(5)  # an odd number of three-step launches
+    a.synchronize()
+    s = torch.cuda.ExternalStream(a.stream())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s, capture_error_mode="thread_local"):
+        a.step(10)
+    g.replay()
+    torch.cuda.synchronize()
+    a.step(8)
+    a.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    c.step(33)
+    for d in range(2):
+        np.testing.assert_array_equal(a.populations(d), c.populations(d))

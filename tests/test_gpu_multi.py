@@ -240,3 +240,47 @@ def test_bands_of_twelve_rows_and_a_remainder(lbm, cuda_ok, oracle_mod, storage,
         o.step(n)
     same(lat, o)
     lat.close()
+
+
+@pytest.mark.parametrize("storage,sr,nx,ny", [(0, None, 200, 64), (0, None, 121, 3400), (1, 9, 200, 64)])
+@pytest.mark.parametrize("before", [4, 7])
+def test_a_callers_graph_survives_other_steps(lbm, cuda_ok, oracle_mod, storage, sr, nx, ny, before):
+    """Ten steps and a population read captured by the caller, replayed around
+    plain calls: the graph keeps reading the rest plane that holds the state
+    (before: an odd or an even number of three-step launches precedes it)."""
+    import torch
+    from lbm_gb300 import load_library
+    lat, o = pair(lbm, oracle_mod, nx, ny, storage, 5, False, sr)
+    s = torch.cuda.Stream()
+    lat.set_stream(s.cuda_stream)
+    lat.iterate(before)
+    o.step(before)
+    lat.populations()
+    out = torch.zeros(9, ny, nx, device="cuda")
+    torch.cuda.synchronize()
+
+    def ten():
+        lat.iterate(10)
+        lbm._check(load_library().lbm_read_populations_device(lat.handle, ctypes.c_void_p(out.data_ptr())))
+
+    s.synchronize()
+    ten()  # the state is now as a replay leaves it
+    o.step(10)
+    lat.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s, capture_error_mode="thread_local"):
+        ten()
+    for _ in range(2):
+        g.replay()
+        torch.cuda.synchronize()
+        o.step(10)
+        np.testing.assert_array_equal(out.cpu().numpy(), o.state()[0].astype(np.float32))
+    lat.iterate(10)
+    lat.populations()
+    lat.synchronize()
+    o.step(10)
+    g.replay()
+    torch.cuda.synchronize()
+    o.step(10)
+    same(lat, o)
+    lat.close()

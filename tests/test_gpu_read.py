@@ -1,4 +1,4 @@
-"""Populations read between steps from the fused representation: the values of
+"""Populations read between steps, materialised in the same pass: the values of
 the materialised state, bit for bit, and no trace in the steps that follow."""
 import numpy as np
 import pytest
@@ -30,8 +30,7 @@ def test_read_between_steps_equals_the_materialised_state(lbm, cuda_ok, storage,
         a.iterate(n)
         b.iterate(n)
         pulled = a.populations(f64=storage == 3)
-        a.checkpoint()  # leaves the pre-collision state in memory
-        np.testing.assert_array_equal(a.populations(f64=storage == 3), pulled)
+        np.testing.assert_array_equal(a.populations(f64=storage == 3), pulled)  # from memory
     a.iterate(2)
     a.populations()
     a.iterate(3)
