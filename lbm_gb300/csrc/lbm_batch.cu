@@ -275,7 +275,7 @@ struct lbm_batch {
   CUtensorMap* d_maps = nullptr;  // two per domain: the 8 planes of each buffer set
   int4* d_mtiles = nullptr;       // tiles of the three-step launches
   int nmtiles = 0, rest_i = 0;    // their number; the rest planes that hold the state
-  bool captured = false;          // the caller captured steps: one step per launch from then on, as the
+  bool captured = false;          // the caller captured work: one step per launch from then on, as the
                                   // captured launches hold the addresses of the rest planes
   int* d_counter = nullptr;  // one ticket counter per step of a captured graph
   int counters_cap = 0;
@@ -340,6 +340,18 @@ void drop_graphs(lbm_batch* b) {
       cudaGraphExecDestroy(g);
       g = nullptr;
     }
+}
+
+// Whether the caller is capturing the batch's stream; remembered in `captured`.
+int note_capture(lbm_batch* b) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  BCK(cudaStreamIsCapturing(b->stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) {
+    b->captured = true;
+    if (b->cfg.multi) drop_graphs(b);
+    b->cfg.multi = false;
+  }
+  return LBM_OK;
 }
 
 // Tile table for the current configuration, longest tiles first.
@@ -754,6 +766,8 @@ int lbm_batch_set_mask(lbm_batch* b, uint32_t domain, const uint8_t* mask) {
 
 int lbm_batch_init_equilibrium(lbm_batch* b, float noise_amp, uint64_t seed) {
   if (!b) return bfail(LBM_ERR_ARG, "null batch");
+  int rc = note_capture(b);
+  if (rc) return rc;
   auto go = [&](auto tag) -> int {
     using St = decltype(tag);
     using S = typename St::S;
@@ -768,8 +782,7 @@ int lbm_batch_init_equilibrium(lbm_batch* b, float noise_amp, uint64_t seed) {
     BCK(cudaGetLastError());
     return LBM_OK;
   };
-  int rc = dispatch_st(b->storage, go);
-  if (rc) return rc;
+  if ((rc = dispatch_st(b->storage, go))) return rc;
   b->launches += b->count;
   BCK(cudaMemsetAsync(b->d_flag, 0, 4, b->stream));  // a fresh start clears the error flags
   b->cur = 0;
@@ -781,14 +794,8 @@ int lbm_batch_init_equilibrium(lbm_batch* b, float noise_amp, uint64_t seed) {
 
 int lbm_batch_step(lbm_batch* b, uint32_t n) {
   if (!b) return bfail(LBM_ERR_ARG, "null batch");
-  int rc;
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  BCK(cudaStreamIsCapturing(b->stream, &capturing));
-  if (capturing != cudaStreamCaptureStatusNone) {
-    b->captured = true;
-    if (b->cfg.multi) drop_graphs(b);
-    b->cfg.multi = false;
-  }
+  int rc = note_capture(b);
+  if (rc) return rc;
   for (uint32_t k = 0; k < n;) {
     const uint32_t left = n - k;
     const bool last = left == 1;

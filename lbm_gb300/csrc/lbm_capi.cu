@@ -217,10 +217,20 @@ template <class F> int dispatch_storage(int storage, F&& f) {
   return fail(LBM_ERR_ARG, "bad storage %d", storage);
 }
 
+// Whether the caller is capturing the handle's stream; remembered in `captured`.
+int note_capture(lbm_sim* s, bool* now = nullptr) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (s->stream != nullptr) CK(cudaStreamIsCapturing(s->stream, &st));
+  if (st != cudaStreamCaptureStatusNone) s->captured = true;
+  if (now) *now = st != cudaStreamCaptureStatusNone;
+  return LBM_OK;
+}
+
 // Re-express every stored 16-bit word (both sets, rest plane) from reference
 // `from` to reference `to`; f32 / f64 storage is unaffected.
 int rebase(lbm_sim* s, const StoreRef& from, const StoreRef& to) {
   if (s->storage != STORE_F16 && s->storage != STORE_BF16) return LBM_OK;
+  if (int rc = note_capture(s)) return rc;
   dim3 grid((s->L.nx + kBlockX - 1) / kBlockX, s->L.ny);
   auto launch = [&](auto tag) -> int {
     using St = decltype(tag);
@@ -305,15 +315,6 @@ void default_walls(lbm_sim* s) {
   }
 }
 
-// Whether the caller is capturing the handle's stream; remembered in `captured`.
-int note_capture(lbm_sim* s, bool* now = nullptr) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (s->stream != nullptr) CK(cudaStreamIsCapturing(s->stream, &st));
-  if (st != cudaStreamCaptureStatusNone) s->captured = true;
-  if (now) *now = st != cudaStreamCaptureStatusNone;
-  return LBM_OK;
-}
-
 // Bring the reference's pre-collision state S_k into buffer `cur`.
 int materialise(lbm_sim* s) {
   if (s->materialised) return LBM_OK;
@@ -354,6 +355,7 @@ int reset_clock(lbm_sim* s) {
 
 int launch_init(lbm_sim* s, double rho, double ux, double uy, double amp, uint64_t seed, int single,
                 long long single_cell, const float* noise_d = nullptr) {
+  if (int rc = note_capture(s)) return rc;
   dim3 grid((s->L.nx + kBlockX - 1) / kBlockX, s->L.ny);
   auto launch = [&](auto tag) -> int {
     using St = decltype(tag);
@@ -892,6 +894,7 @@ int lbm_set_viscosity(lbm_sim* s, float nu) {
 // field reset, the stored words are first re-expressed against the new one.
 int lbm_set_inlet_velocity(lbm_sim* s, float ux, int reset_field) {
   CHECK_SIM(s);
+  if (int rc = note_capture(s)) return rc;
   if (reset_field) {
     s->u_in = ux;
     return launch_init(s, 1.0, ux, 0.0, 0.0, 0, -1, -1);
@@ -1382,9 +1385,10 @@ int lbm_read_populations_device(lbm_sim* s, float* device_out) { return read_pop
 static int write_pops(lbm_sim* s, const void* in, bool f64) {
   CHECK_SIM(s);
   if (!in) return fail(LBM_ERR_ARG, "in is null");
+  int rc = note_capture(s);
+  if (rc) return rc;
   // a page-locked `in` is read by the kernel itself; other memory is staged
   const void* src = mapped_host(in);
-  int rc = LBM_OK;
   if (!src) {
     rc = copy_from_host(s, s->staging_d, in, (size_t)9 * s->L.nx * s->L.ny * (f64 ? 8 : 4));
     if (rc) return rc;

@@ -284,3 +284,29 @@ def test_a_callers_graph_survives_other_steps(lbm, cuda_ok, oracle_mod, storage,
     o.step(10)
     same(lat, o)
     lat.close()
+
+
+def test_a_callers_captured_inlet_change_survives_other_steps(lbm, cuda_ok, oracle_mod):
+    """An inlet change captured by the caller and replayed after plain steps
+    sets the column of the rest plane that holds the state."""
+    import torch
+    lat, o = pair(lbm, oracle_mod, 200, 64, 0, 5, False, None)
+    s = torch.cuda.Stream()
+    lat.set_stream(s.cuda_stream)
+    lat.iterate(10)
+    lat.populations()
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=s, capture_error_mode="thread_local"):
+        lat.set_inlet_velocity(0.12)
+    lat.iterate(13)
+    lat.populations()
+    lat.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    lat.iterate(7)
+    o.step(23)
+    o.set_inlet(0.12)
+    o.step(7)
+    same(lat, o)
+    lat.close()
