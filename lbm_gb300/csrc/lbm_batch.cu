@@ -231,8 +231,11 @@ __global__ void __launch_bounds__(32, kMultiOcc)
     m.rest_out = (S*)doms[T.x].rest[1 - rest_i];
     m.one = one;
   }
+  const CUtensorMap* map = maps + 2 * T.x + src_i;
   __syncwarp();
-  multi_dispatch<St, SR>(m, maps + 2 * T.x + src_i, T.y, T.z, T.w, smem, full);
+  if (elect_one()) acquire_map(map);  // the lane that issues every copy (the election is the same each time)
+  __syncwarp();
+  multi_dispatch<St, SR>(m, map, T.y, T.z, T.w, smem, full);
 }
 
 struct DomainHost {

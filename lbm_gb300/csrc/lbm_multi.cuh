@@ -314,6 +314,14 @@ __device__ __forceinline__ void tensor_g2s(uint32_t dst, const CUtensorMap* map,
       : "memory");
 }
 
+// Before the first copy through a tensor map that lies in global memory and was
+// written by a copy: later tensor copies of this lane see the map's present
+// contents, not what a freed map at the same address held.  (A map passed as a
+// __grid_constant__ argument needs none.)
+__device__ __forceinline__ void acquire_map(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
+
 template <class S, class C> struct MultiArgs {
   StepArgs<S, C> a;
   S* rest_out;

@@ -333,3 +333,30 @@ def test_a_callers_graph_of_batch_steps_survives_other_steps(lbm, cuda_ok):
     c.step(33)
     for d in range(2):
         np.testing.assert_array_equal(a.populations(d), c.populations(d))
+
+
+@pytest.mark.parametrize("storage", [0, 1])
+def test_a_batch_in_the_place_of_a_destroyed_one(lbm, cuda_ok, oracle_mod, storage):
+    """Batches created one after another where the last one was destroyed (the
+    allocator tends to give the same addresses again), of other domain sizes and
+    numbers: three-step launches read the new batch's planes, every domain equal to
+    its oracle run."""
+    from lbm_gb300 import batch
+    P = oracle_mod
+    rng = np.random.default_rng(9)
+    for k, sizes in enumerate([[(700, 320), (640, 350)], [(320, 700), (350, 640)], [(61, 4000), (123, 2000)],
+                               [(700, 320), (128, 1750)], [(180, 160)] * 16]):
+        nx, ny = (np.array(v, np.uint32) for v in zip(*sizes))
+        omega = np.full(len(sizes), 1.4, np.float32)
+        u_in = rng.uniform(0.02, 0.07, len(sizes)).astype(np.float32)
+        with batch.Batch(nx, ny, omega, u_in, storage) as b:
+            assert b.info()[1] >= 400000
+            b.init_equilibrium(1e-2, k)
+            masks = [(rng.random((int(y), int(x))) < 0.1).astype(np.uint8) for x, y in zip(nx, ny)]
+            for d, m in enumerate(masks):
+                b.set_mask(d, m)
+            b.step(8)
+            for d, m in enumerate(masks):
+                o = oracle_for(P, b, d, storage, m, 1e-2, k)
+                o.step(8)
+                assert_domain(b, d, o)
