@@ -562,7 +562,10 @@ __device__ __forceinline__ void multi_tile(const MultiArgs<typename St::S, typen
       for (int i = max(0, issued - NS); i < issued; i++) mbar_wait(smem_addr(&full[i % NS]), (uint32_t)(i / NS) & 1u);
       break;
     }
-    if (divide || __all_sync(0xffffffffu, (range.ok_x() || !cell[0]) && (range.ok_y() || !cell[1]))) break;
+    // the halo lanes' cells count too: their neighbours are stored (columns 0
+    // and outside the lattice hold whatever was pulled and feed nothing)
+    const bool in0 = !EDGE || (x0 >= 1 && x0 < L.nx), in1 = !EDGE || (x0 >= 0 && x0 + 1 < L.nx);
+    if (divide || __all_sync(0xffffffffu, (range.ok_x() || !in0) && (range.ok_y() || !in1))) break;
     rho_sum = 0.0f;
     __syncwarp();
     if (lane == 0)
