@@ -72,9 +72,19 @@ constexpr long long kPadCells = 4096;
 //     800, bf16: three at once 6.5 us a step against 7.5, alone 10.2 against
 //     13.1; 768 x 768: 5.0 against 4.5, alone 8.3 against 8.3); between the two
 //     kernels' ranges the one-step kernels stay.
-// The closure's steps run in k_step_tile: in f32 on any lattice, in 16-bit
-// storage on small ones.
+// The closure's steps run in k_step_tile on small lattices, else one per
+// launch: k_step_tile is the faster one alone up to half a million cells, but
+// beside other lattices it falls behind earlier, and the lines lie where that
+// costs 5 %.  us per step, alone / three at once, against the one-step kernel:
+// f32 512 x 256 2.78 / 1.77 against 4.43 / 2.16, 780 x 520 6.97 / 5.50 against
+// 9.13 / 5.67, 1024 x 512 7.90 / 7.01 against 8.93 / 6.43, 2048 x 1024 28.6 / 26.7
+// against 29.3 / 24.4, 4096 x 2048 107 / 105 against 103 / 95; f16 384 x 384 3.86 /
+// 2.16 against 5.22 / 2.35, 450 x 400 4.02 / 2.50 against 5.33 / 2.45, 512 x 400
+// 4.06 / 2.78 against 5.24 / 2.45; bf16 with stochastic rounding 450 x 400 4.60 /
+// 2.70 against 5.84 / 2.65, 610 x 400 5.34 / 3.59 against 6.41 / 3.28.
 constexpr uint64_t kTileCells16 = 250000;     // k_step_tile below, 16-bit storage
+constexpr uint64_t kClosureCells32 = 450000;  // closure: k_step_tile below, f32
+constexpr uint64_t kClosureCells16 = 190000;  // 16-bit storage
 constexpr uint64_t kMultiCells32 = 400000;    // k_step_multi from here: f32 (k_step_tile below)
 constexpr uint64_t kMultiCells16 = 250000;    // 16-bit storage
 constexpr uint64_t kMultiCellsSr = 900000;    // 16-bit storage with stochastic rounding
@@ -570,9 +580,10 @@ bool pair_ok(const lbm_sim* s) {
 enum { THREE_NONE, THREE_TILE, THREE_ROWS };
 int three_kernel(const lbm_sim* s) {
   const uint64_t cells = (uint64_t)s->L.nx * s->L.ny;
-  if (s->storage == STORE_F32) return s->closure_on || cells < kMultiCells32 ? THREE_TILE : THREE_ROWS;
+  if (s->closure_on)
+    return cells < (s->storage == STORE_F32 ? kClosureCells32 : kClosureCells16) ? THREE_TILE : THREE_NONE;
+  if (s->storage == STORE_F32) return cells < kMultiCells32 ? THREE_TILE : THREE_ROWS;
   if (cells < kTileCells16) return THREE_TILE;
-  if (s->closure_on) return THREE_NONE;
   return cells >= (s->sr_on ? kMultiCellsSr : kMultiCells16) ? THREE_ROWS : THREE_NONE;
 }
 // Whether a call may take three steps in one launch: the lattice's default

@@ -310,3 +310,21 @@ def test_a_callers_captured_inlet_change_survives_other_steps(lbm, cuda_ok, orac
     o.step(7)
     same(lat, o)
     lat.close()
+
+
+@pytest.mark.parametrize("storage,nx,ny,three", [(0, 700, 640, True), (0, 1024, 512, False), (1, 450, 400, True),
+                                                 (2, 512, 400, False)])
+def test_closure_steps_share_launches_on_small_lattices_only(lbm, cuda_ok, storage, nx, ny, three):
+    """With the closure on, three steps share a launch on small lattices; larger
+    ones step one by one, which is faster there."""
+    L = lbm.load_library()
+    lat = lbm.Lattice(nx, ny, 1.4, lbm.EDGE_CHANNEL, storage)
+    w = np.zeros(19969, np.float32)
+    lbm._check(L.lbm_closure_set_weights(lat.handle, w.ctypes.data, w.size))
+    lbm._check(L.lbm_closure_enable(lat.handle, 0.2))
+    lat.iterate(2)
+    lbm._check(L.lbm_closure_infer(lat.handle))
+    before = lat.launch_count()
+    lat.iterate(20)
+    assert lat.launch_count() - before == (8 if three else 20)
+    lat.close()
