@@ -559,7 +559,7 @@ int capture_graph(lbm_batch* b) {
     cudaGraphExecDestroy(out);
     out = nullptr;
   }
-  const int cur0 = b->cur;
+  const int cur0 = b->cur, rest0 = b->rest_i;
   const uint64_t steps0 = b->steps, launches0 = b->launches;
   int rc = advance_clock(b);  // the graph's launches count from the clock as it stands
   if (rc) return rc;
@@ -572,10 +572,14 @@ int capture_graph(lbm_batch* b) {
   if (!rc) rc = advance_clock(b);  // recorded: every replay advances the clock
   b->clock_pending = 0;
   cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-  b->cur = cur0;  // capture recorded the launches without running them (the rest planes end where they began)
+  b->cur = cur0;  // capture recorded the launches without running them
+  b->rest_i = rest0;  // (a whole run leaves the rest planes as they were, one cut short by an error need not)
   b->steps = steps0;
   b->launches = launches0;
-  if (rc) return rc;
+  if (rc) {
+    if (e == cudaSuccess) cudaGraphDestroy(g);
+    return rc;
+  }
   if (e != cudaSuccess) return bfail(LBM_ERR_CUDA, "stream capture: %s", cudaGetErrorString(e));
   e = cudaGraphInstantiate(&out, g, 0);
   cudaGraphDestroy(g);
