@@ -7,9 +7,12 @@
  * bounce-back from its own mask, its own omega.
  * lbm_batch_step advances every domain together: one persistent kernel
  * launch per step over a table of (domain, 256-column strip, row band) tiles,
- * or, for batches of 400,000 cells or more unless a schedule was fixed by hand
- * or the autotuner found otherwise, one launch per three steps; runs of 20 (18)
- * steps are replayed from a CUDA graph captured on first use.
+ * or, for batches of 400,000 cells or more (1,600,000 with stochastic rounding)
+ * unless a schedule was fixed by hand or the autotuner found otherwise, one
+ * launch per three steps; runs of 20 (18) steps are replayed from a CUDA graph
+ * captured on first use.  Once the caller has captured work on a batch's stream,
+ * the batch keeps to one step per launch: the captured launches hold the
+ * addresses of the buffers that were current then.
  * Results are bit-identical to advancing each domain through lbm_sim.
  *
  * Storage: LBM_STORE_F32, LBM_STORE_F16, LBM_STORE_BF16.  Every call is
@@ -73,7 +76,8 @@ int lbm_batch_conservation(lbm_batch* batch, double* out);
  * default) or, for f16 / bf16 batches, LBM_ROUND_STOCHASTIC.  Domain d then
  * rounds exactly as a single lattice of its size with seed `seed + d`; the
  * step index is the batch's.  LBM_ERR_ARG for stochastic rounding of an
- * f32 batch. */
+ * f32 batch.  What the autotuner found holds for the mode that it ran in; a
+ * schedule fixed by hand holds in both. */
 int lbm_batch_set_rounding(lbm_batch* batch, int mode, uint32_t seed);
 int lbm_batch_get_rounding(const lbm_batch* batch, int* mode, uint32_t* seed);
 

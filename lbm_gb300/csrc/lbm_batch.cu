@@ -290,6 +290,9 @@ struct lbm_batch {
   bool materialised = true, moments_valid = false;
   uint64_t steps = 0, launches = 0, cells = 0;
   Config cfg;
+  // per rounding mode: three steps per launch as fixed by hand or found by the
+  // autotuner in that mode (0, 1), or the default (-1)
+  int multi_choice[2] = {-1, -1};
   int grid = 0;  // persistent CTAs
   cudaGraphExec_t graph[4] = {};  // a run of steps from each buffer and rest-plane parity
   std::string report;
@@ -396,8 +399,10 @@ size_t multi_smem(int storage) {
   return storage == STORE_F32 ? (size_t)MultiGeom<float>::kStages * MultiGeom<float>::kBytes
                               : (size_t)MultiGeom<__half>::kStages * MultiGeom<__half>::kBytes;
 }
-bool multi_default(const lbm_batch* b) {
-  return !b->captured && b->cells >= (b->sr_on ? kMultiCellsSr : kMultiCells);
+// Whether calls take three steps per launch in the present rounding mode.
+bool use_multi(const lbm_batch* b) {
+  const int choice = b->multi_choice[b->sr_on];
+  return !b->captured && (choice < 0 ? b->cells >= (b->sr_on ? kMultiCellsSr : kMultiCells) : choice != 0);
 }
 
 // Tensor maps and tiles of the three-step launches: bands of 8 to 24 rows, as
@@ -726,7 +731,7 @@ int lbm_batch_create(uint32_t count, const uint32_t* nx, const uint32_t* ny, con
   if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) return cleanup(LBM_ERR_CUDA, "setup", e);
   int rc = ensure_counters(b);
   if (!rc) rc = build_multi(b);
-  b->cfg.multi = multi_default(b);
+  b->cfg.multi = use_multi(b);
   if (!rc) rc = configure(b);
   if (!rc) rc = lbm_batch_init_equilibrium(b, 0.0f, 0);
   if (rc) {
@@ -945,7 +950,7 @@ int lbm_batch_set_rounding(lbm_batch* b, int mode, uint32_t seed) {
   b->sr_seed = b->sr_on ? seed : 0u;
   int rc = reset_clock(b);  // the clock counts on from the current step
   if (rc) return rc;
-  b->cfg.multi = b->cfg.multi && multi_default(b);
+  b->cfg.multi = use_multi(b);
   return configure(b);  // the kernel, its occupancy and the captured graphs change
 }
 
@@ -963,6 +968,7 @@ int lbm_batch_set_schedule(lbm_batch* b, int variant, int dynamic, const int* ro
   b->cfg.variant = variant;
   b->cfg.dynamic = dynamic;
   b->cfg.multi = false;
+  b->multi_choice[0] = b->multi_choice[1] = 0;
   if (rows_per_bucket)
     for (int i = 0; i < kBuckets; i++) b->cfg.rows[i] = std::max(1, rows_per_bucket[i]);
   return configure(b);
@@ -1048,6 +1054,7 @@ int lbm_batch_autotune(lbm_batch* b, uint32_t steps_per_trial, char* report, siz
   int rc = b->captured ? LBM_OK : trial("three_steps", &best, &best_cfg);
   if (rc) return rc;
   b->cfg = best_cfg;
+  if (!b->captured) b->multi_choice[b->sr_on] = b->cfg.multi ? 1 : 0;
   rc = configure(b);
   if (rc) return rc;
   const int NS = kVariants[b->cfg.variant][0], CPT = kVariants[b->cfg.variant][1];
