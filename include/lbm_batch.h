@@ -93,8 +93,9 @@ int lbm_batch_get_rounding(const lbm_batch* batch, int* mode, uint32_t* seed);
 int lbm_batch_set_schedule(lbm_batch* batch, int variant, int dynamic, const int* rows_per_bucket);
 
 /* Time the candidate schedules on this batch (each for steps_per_trial steps
- * after a warm-up; the state advances meanwhile) and keep the fastest.  The
- * trials and the choice are written as JSON into report (report_len bytes,
+ * after a warm-up; the state advances meanwhile) and keep the fastest; one
+ * against three steps per launch is decided over the replayed runs of long calls
+ * (two of them, 36 or 40 steps, or more up to steps_per_trial).  The trials and the choice are written as JSON into report (report_len bytes,
  * truncated; may be NULL). */
 int lbm_batch_autotune(lbm_batch* batch, uint32_t steps_per_trial, char* report, size_t report_len);
 

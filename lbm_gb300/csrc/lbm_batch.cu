@@ -592,6 +592,19 @@ int capture_graph(lbm_batch* b) {
   return LBM_OK;
 }
 
+// Replay a run of graph_steps steps from the current parity (an even number of
+// steps: the buffer parity is unchanged), recorded first where there is none.
+int replay_run(lbm_batch* b) {
+  int rc;
+  if (!graph_of(b) && (rc = capture_graph(b))) return rc;
+  if ((rc = advance_clock(b))) return rc;
+  BCK(cudaGraphLaunch(graph_of(b), b->stream));
+  const int run = graph_steps(b);
+  b->launches += (b->cfg.multi ? run / kMultiSteps : run) + (b->sr_on ? 1 : 0);
+  b->steps += run;
+  return LBM_OK;
+}
+
 int materialise_all(lbm_batch* b) {
   if (b->materialised) return LBM_OK;
   const int dst = 1 - b->cur;
@@ -813,11 +826,7 @@ int lbm_batch_step(lbm_batch* b, uint32_t n) {
     const bool last = left == 1;
     const uint32_t run = (uint32_t)graph_steps(b);
     if (!b->materialised && !last && left > run) {
-      if (!graph_of(b) && (rc = capture_graph(b))) return rc;
-      if ((rc = advance_clock(b))) return rc;
-      BCK(cudaGraphLaunch(graph_of(b), b->stream));
-      b->launches += (b->cfg.multi ? run / kMultiSteps : run) + (b->sr_on ? 1 : 0);
-      b->steps += run;  // an even number: the buffer parity is unchanged
+      if ((rc = replay_run(b))) return rc;
       k += run;
       continue;
     }
@@ -974,20 +983,26 @@ int lbm_batch_set_schedule(lbm_batch* b, int variant, int dynamic, const int* ro
   return configure(b);
 }
 
-// Times `steps` steps of the current configuration (after one warm-up step);
-// the state advances by steps + 1.
-static int time_config(lbm_batch* b, int steps, float* ms) {
+// Times `steps` steps of the current configuration (after one warm-up step), or
+// whole replayed runs of at least as many (after one more); milliseconds per step.
+static int time_config(lbm_batch* b, int steps, bool runs, float* ms) {
   int rc = configure(b);
   if (rc) return rc;
   if ((rc = lbm_batch_step(b, 1))) return rc;
+  const int run = graph_steps(b), count = std::max(2, (steps + run - 1) / run);
+  if (runs && (rc = replay_run(b))) return rc;  // recorded outside the timing
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, b->stream);
-  rc = lbm_batch_step(b, (uint32_t)steps);
+  if (runs)
+    for (int i = 0; i < count && !rc; i++) rc = replay_run(b);
+  else
+    rc = lbm_batch_step(b, (uint32_t)steps);
   cudaEventRecord(e1, b->stream);
   cudaEventSynchronize(e1);
   cudaEventElapsedTime(ms, e0, e1);
+  *ms /= runs ? count * run : steps;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (rc) return rc;
@@ -1006,13 +1021,13 @@ int lbm_batch_autotune(lbm_batch* b, uint32_t steps_per_trial, char* report, siz
   std::string rep = "{\"trials\": [";
   char buf[512];
   bool first = true;
-  auto trial = [&](const char* stage, float* best, Config* keep) -> int {
+  auto trial = [&](const char* stage, float* best, Config* keep, bool runs = false) -> int {
     float ms = 0.0f;
-    int rc = time_config(b, T, &ms);
+    int rc = time_config(b, T, runs, &ms);
     if (rc) return rc;
     snprintf(buf, sizeof buf, "%s{\"stage\": \"%s\", \"variant\": %d, \"dynamic\": %d, \"rows\": [%d, %d, %d], "
              "\"steps_per_launch\": %d, \"ms_per_step\": %.5f}", first ? "" : ", ", stage, b->cfg.variant, b->cfg.dynamic,
-             b->cfg.rows[0], b->cfg.rows[1], b->cfg.rows[2], b->cfg.multi ? kMultiSteps : 1, ms / T);
+             b->cfg.rows[0], b->cfg.rows[1], b->cfg.rows[2], b->cfg.multi ? kMultiSteps : 1, ms);
     rep += buf;
     first = false;
     if (ms < *best) {
@@ -1048,14 +1063,21 @@ int lbm_batch_autotune(lbm_batch* b, uint32_t steps_per_trial, char* report, siz
       if (rc) return rc;
     }
   }
-  // stage 3: three steps per launch, the schedule above for the other steps
+  // stage 3: three steps per launch, the schedule above for a call's last steps.
+  // Both forms are timed over the runs that long calls replay: a call of
+  // steps_per_trial steps ends with one to three single steps in either form,
+  // and a short one holds no others.
   b->cfg = best_cfg;
-  b->cfg.multi = !b->captured;
-  int rc = b->captured ? LBM_OK : trial("three_steps", &best, &best_cfg);
-  if (rc) return rc;
+  if (!b->captured) {
+    best = 3.4e38f;
+    int rc = trial("one_step", &best, &best_cfg, true);
+    if (rc) return rc;
+    b->cfg.multi = true;
+    if ((rc = trial("three_steps", &best, &best_cfg, true))) return rc;
+  }
   b->cfg = best_cfg;
   if (!b->captured) b->multi_choice[b->sr_on] = b->cfg.multi ? 1 : 0;
-  rc = configure(b);
+  int rc = configure(b);
   if (rc) return rc;
   const int NS = kVariants[b->cfg.variant][0], CPT = kVariants[b->cfg.variant][1];
   snprintf(buf, sizeof buf, "], \"chosen\": {\"ring_stages\": %d, \"cells_per_thread\": %d, \"strip_columns\": %d, "
@@ -1063,7 +1085,7 @@ int lbm_batch_autotune(lbm_batch* b, uint32_t steps_per_trial, char* report, siz
            "\"rows_per_band\": {\"ny<=128\": %d, \"ny<=256\": %d, \"ny>256\": %d}, \"ms_per_step\": %.5f, "
            "\"persistent_ctas\": %d, \"tiles\": %d}}",
            NS, CPT, strip_of(b->cfg.variant, b->storage), b->cfg.dynamic == 1 ? "dynamic" : (b->cfg.dynamic == 2 ? "static_one_ring" : "static_longest_first"), b->cfg.multi ? kMultiSteps : 1, b->cfg.rows[0], b->cfg.rows[1], b->cfg.rows[2],
-           best / T, b->grid, b->ntiles);
+           best, b->grid, b->ntiles);
   rep += buf;
   b->report = rep;
   if (report && report_len) {

@@ -1,6 +1,7 @@
 """The host code of lbm_batch.cu against stand-ins for the CUDA calls that it
 makes (no GPU): a recording that an error cuts short leaves the batch as it was;
-the steps per launch follow the rounding mode and what was chosen for it."""
+the steps per launch follow the rounding mode and what was chosen for it; the
+autotuner's choice between one and three steps does not depend on its trials' length."""
 import os
 import subprocess
 
@@ -15,7 +16,7 @@ HARNESS = r"""
 #include <cstring>
 // launches of the one-step and of the three-step kernel (the first takes 14
 // arguments' worth of block, the second one warp) are told apart by block size
-static int launches_left = 1 << 30, destroyed, singles, triples, recorded[2], recording;
+static int launches_left = 1 << 30, destroyed, singles, triples, recorded[2], recording, captures;
 template <class F> static cudaError_t fake_launch(F, dim3, dim3 block, void**, size_t, cudaStream_t) {
   if (launches_left-- <= 0) return cudaErrorLaunchFailure;
   (recording ? recorded[block.x == 32] : block.x == 32 ? triples : singles)++;
@@ -30,6 +31,7 @@ static cudaError_t fake_begin(cudaStream_t, cudaStreamCaptureMode) {
 static cudaError_t fake_end(cudaStream_t, cudaGraph_t* g) { recording = 0; *g = nullptr; return cudaSuccess; }
 static cudaError_t fake_instantiate(cudaGraphExec_t* out, cudaGraph_t, unsigned long long) {
   *out = (cudaGraphExec_t) new Run{recorded[0], recorded[1]};
+  captures++;
   return cudaSuccess;
 }
 static cudaError_t fake_replay(cudaGraphExec_t g, cudaStream_t) {
@@ -47,12 +49,12 @@ template <class F> static cudaError_t fake_occupancy(int* v, F, int, size_t) { *
 static cudaError_t fake_capturing(cudaStream_t, cudaStreamCaptureStatus* s) { *s = cudaStreamCaptureStatusNone; return cudaSuccess; }
 template <class... A> static cudaError_t fine(A...) { return cudaSuccess; }
 static cudaError_t fake_copy(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t = nullptr) { memcpy(d, s, n); return cudaSuccess; }
-// a clock that moves by each launch's cost
+// a clock that moves by each launch's cost and by each recording's
 static float single_ms = 1.0f, triple_ms = 1.5f, stamps[2];
 static int stamped;
 static cudaError_t fake_event(cudaEvent_t*) { stamped = 0; return cudaSuccess; }
 static cudaError_t fake_record(cudaEvent_t, cudaStream_t) {
-  stamps[stamped++ & 1] = singles * single_ms + triples * triple_ms;
+  stamps[stamped++ & 1] = singles * single_ms + triples * triple_ms + captures * 30.0f;
   return cudaSuccess;
 }
 static cudaError_t fake_elapsed(float* ms, cudaEvent_t, cudaEvent_t) { *ms = stamps[1] - stamps[0]; return cudaSuccess; }
@@ -127,6 +129,18 @@ int main(int argc, char** argv) {
     }
     printf("\n");
   }
+  if (!strcmp(argv[1], "tune"))  // steps per trial: the form chosen where it is the faster one by a tenth
+    for (int form = 1; form <= 3; form += 2) {
+      lbm_batch b;
+      set_up(b, STORE_F32, 500000);
+      triple_ms = form == 3 ? 2.7f : 3.3f;
+      char report[16384];
+      lbm_batch_autotune(&b, (uint32_t)atoi(argv[2]), report, sizeof report);
+      const char* chosen = strstr(report, "chosen");
+      float ms = 0.0f;
+      sscanf(strstr(chosen, "ms_per_step"), "ms_per_step\": %f", &ms);
+      printf("%d %d\n", per_launch(b), (int)(ms * 1000 + 0.5f));
+    }
   fflush(stdout);
   _Exit(0);
 }
@@ -173,3 +187,11 @@ def test_a_recording_cut_short_leaves_the_rest_planes(harness):
 ])
 def test_steps_per_launch_follow_the_rounding_mode(harness, cells, calls, want):
     assert harness("rounding", cells, *calls.split()) == [want]
+
+
+@pytest.mark.parametrize("steps", [1, 2, 3, 8, 18, 19, 20, 21, 40, 100])
+def test_the_autotuner_finds_the_faster_form_at_any_trial_length(harness, steps):
+    """A three-step launch that costs a tenth less (more) than three single ones:
+    short trials, in which few or no steps share a launch, and trials during which
+    a run would have to be recorded choose it (not) like long ones."""
+    assert harness("tune", steps) == [[1, 1000], [3, 900]]
