@@ -108,8 +108,9 @@ int lbm_get_stream(const lbm_sim* sim, void** cuda_stream);
  * for kernel 1, 1 for kernel 0 and a band floor of 2 rows for the staged
  * kernels; f64 storage always uses kernel 0.  Until this is called, lbm_step
  * takes three steps per launch where it can (channel mode below f64) and two
- * cells per thread in reference mode; the chosen kernel then takes every step
- * by itself.  No counterpart in the reference, whose dispatch is fixed at
+ * cells per thread in reference mode; the chosen kernel, the defaults named here
+ * included, then takes every step by itself for the rest of the handle's life,
+ * which is the slower way (f32, 4096 x 2048: half the speed).  No counterpart in the reference, whose dispatch is fixed at
  * 256-wide 1-D workgroups (lbm.rs:102-106). */
 int lbm_set_tuning(lbm_sim* sim, int rows_per_thread, int kernel);
 
@@ -233,7 +234,11 @@ int lbm_step_rows(lbm_sim* sim, uint32_t y0, uint32_t y1, int flags);
  * number of steps, from a state that has taken at least one step since its
  * last initialisation or edit (that step collides in place), and the
  * graph can be replayed any number of times.  The host-side step count
- * advances once, by the recorded steps, not per replay. */
+ * advances once, by the recorded steps, not per replay.  Once the caller has
+ * captured steps, reads, an initialisation, an inlet change or an upload of a
+ * lattice, its later steps are one per launch, for the rest of its life: the
+ * captured launches hold the address of the rest plane that was current then,
+ * and three-step launches would put the state into another. */
 int lbm_set_graphs(lbm_sim* sim, int enable);
 
 /* Wait for queued work; returns LBM_ERR_STATE if a step saw a non-finite density. */

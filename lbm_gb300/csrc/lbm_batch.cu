@@ -11,7 +11,7 @@
 // to use is chosen by lbm_batch_autotune, which times the candidates on the
 // batch itself.  Batches of kMultiCells or more take three steps per launch
 // (k_batch_multi, one warp per tile of 60 columns) and use the staged step for
-// a call's last ones.
+// a call's last ones, unless the autotuner finds that slower.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdarg>
@@ -53,7 +53,14 @@ constexpr long long kPad = 4096;  // elements of padding around every buffer (ha
 constexpr int kBuckets = 3;       // domain-height buckets: <= 128, <= 256, taller
 constexpr int kBlock = 128;
 // Batches of at least this many cells start with three-step launches
-// (stochastic rounding: the second figure), as single lattices do.
+// (stochastic rounding: the second figure).  us per step of 100-step calls, one
+// batch alone / three at once, against the best staged schedule that the
+// autotuner found: 8 domains of 400,000 cells together f32 7.7 / 4.3 against 21.0
+// / 9.3, f16 6.7 / 3.3 against 20.7 / 8.5; 16 domains of 1.2 M cells f32 12.8 /
+// 12.4 against 28.9 / 15.9, f16 10.9 / 10.2 against 27.7 / 15.0; 8 domains of 1.6 M
+// cells with stochastic rounding (f16) 13.5 / 12.8 against 28.5 / 17.3.  Below the
+// lines three steps were faster as well, down to 100,000 cells (16 domains, f32 6.3
+// / 2.5 against 9.8 / 4.0); there the autotuner finds them.
 constexpr uint64_t kMultiCells = 400000, kMultiCellsSr = 1600000;
 
 int bucket_of(int ny) { return ny <= 128 ? 0 : (ny <= 256 ? 1 : 2); }
@@ -406,7 +413,7 @@ bool use_multi(const lbm_batch* b) {
 }
 
 // Tensor maps and tiles of the three-step launches: bands of 8 to 24 rows, as
-// many as one wave of CTAs takes (the single lattice's rule over all domains).
+// many as one wave of CTAs takes over all domains, evened out in each domain.
 int build_multi(lbm_batch* b) {
   std::vector<CUtensorMap> maps(2 * (size_t)b->count);
   int sms = 0;

@@ -4,7 +4,9 @@
 // floating-point operations, so the one-step kernel runs at the copy
 // bandwidth with the arithmetic units mostly idle.  This kernel reads the
 // state once, takes kMultiSteps steps on chip and writes it once: a third of
-// the traffic per step, for 3 % redundant rows and 7 % redundant columns.
+// the traffic per step.  The price is cells advanced twice: the levels of a band
+// of h rows cover h + 4, h + 2 and h rows, 2 / h more (8 % at 24 rows, 17 % at
+// 12, 25 % at 8), and 64 columns are advanced for 60 stored (7 %).
 //
 // A CTA is one warp, which owns 64 columns, two per lane, and walks down a
 // band of rows by itself: it fills its own ring of staged rows in shared
@@ -44,11 +46,17 @@ constexpr int kMultiOcc = 16;                       // CTAs (of one warp) per mu
 
 // a / b for b in a moderate range, correctly rounded, sharing the reciprocal
 // between the quotients of one denominator: y = 1 / b to the nearest (an
-// approximation within one ulp and one Newton step with fused operations, exact
-// but for a mantissa of all ones), then q = a y corrected once by its exact
-// remainder (Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990).  Quotients too small for an exact remainder
-// (|a| < 2^-100) may be off in the last place.
+// approximation within one ulp and one Newton step with fused operations), then
+// q = a y corrected once by its exact remainder (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990).  The
+// method makes one exception for y, a mantissa of all ones (1 - 2^-24 is such a
+// density): 1 / b then lies just above a tie, and the step rounds to the nearest
+// only from an approximation above it.  rcp.approx gives that one: over all 2^23
+// mantissas at eight exponents from 2^-57 to 2^63 every y equalled 1 / b, and
+// sixteen quotients by each equalled a / b.  Quotients too small for an exact
+// remainder (|a| < 2^-100) may be off in the last place; with b of at least
+// 2^-63 they are velocities below 2^-37, added to 1, and only a tie of a later
+// rounding could tell.
 __device__ __forceinline__ float rcp_approx(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

@@ -11,7 +11,11 @@
 // the arithmetic on lattices that fit it, by HBM above.  f32, us per step, against
 // the staged kernel: 256 x 128 3.9 against 6.1, 600 x 400 4.7 against 8.0,
 // 1100 x 700 7.6 against 18.2, 2048 x 1024 26.3 against 40.4, 4096 x 2048 96.6
-// against 158.7 (6090 GB/s).
+// against 158.7 (6090 GB/s).  f16 (bf16 the same within 3 %), alone / three
+// lattices at once: 256 x 128 8.6 / 3.0 against 9.7 / 3.9, 600 x 400 8.1 / 3.2
+// against 11.6 / 6.1, 1100 x 700 9.3 / 4.8 against 28.5 / 13.5, 2048 x 1024 14.1 /
+// 15.4 against 65.8 / 34.9, 4096 x 2048 64 / 61 against 260 / 130, 8192 x 4096 245 /
+// 243 against 993 / 497; with stochastic rounding a tenth more on both sides.
 #pragma once
 #include "lbm_multi.cuh"
 

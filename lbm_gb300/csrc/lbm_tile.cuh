@@ -1,5 +1,5 @@
-// Three steps in one launch for small lattices and for the learned closure
-// (channel mode, f32 and 16-bit storage).
+// Three steps in one launch for small lattices, with or without the learned
+// closure (channel mode, f32 and 16-bit storage).
 //
 // A small lattice's steps are bound by latency: 512 x 256 cells give each
 // multiprocessor 860, and a launch of one step spends most of its 4 us on the
