@@ -774,7 +774,8 @@ def run_ours(args):
                         "median of repeated calls"},
         # against the memory's rate; the kernel itself is held by the FMA pipe and issue
         "roofline": {"bound": "hbm", "limited_by": "FMA pipe and issue", "achieved": round(achieved, 1),
-                     "peak": hbm_peak, "unit": "GB/s", "frac": round(achieved / hbm_peak, 4), "traffic": ncu_traffic("k_step_multi_f32_channel"),
+                     "peak": hbm_peak, "unit": "GB/s", "frac": round(achieved / hbm_peak, 4),
+                     "traffic": ncu_traffic("k_step_multi_f32_channel"),
                      "peak_source": peak_kind, "bytes_per_cell": BYTES_PER_CELL["f32"],
                      "algorithmic_bytes_per_launch": int(BYTES_PER_CELL["f32"] * active),
                      "active_cells": active, "launches_per_call": passes, "steps_per_launch": 3,
